@@ -362,11 +362,16 @@ static int adjoint_fused_t(C *psi, int n, int dtype, const qk_gate *gates, size_
     cut.push_back(ng);
     const size_t nseg = cut.size() - 1;
     std::vector<HostPlan> fwd(nseg), bwd(nseg);
-    PlanOptions fo = default_plan_options(dtype, n), bo = default_adjoint_options(dtype, n);
+    // complex64 sweeps run the general programs both ways: with factored
+    // forward passes the 23-qubit HEA sweep of 10 layers took 18.1 ms against
+    // 17.9, its two-state passes being most of it
+    const PlanOptions fo = dtype == QK_C128 ? factored_plan_options(dtype, n) : default_plan_options(dtype, n);
+    const PlanOptions bo = factored_adjoint_options(dtype, n);
     for (size_t sgi = 0; sgi < nseg; ++sgi) {
-        int rc = build_plan(gates + cut[sgi], cut[sgi + 1] - cut[sgi], n, fo, fwd[sgi]);
-        if (!rc) rc = build_adjoint_plan(gates + cut[sgi], cut[sgi + 1] - cut[sgi], pidx ? pidx + cut[sgi] : nullptr,
-                                         n, bo, bwd[sgi]);
+        const qk_gate *g = gates + cut[sgi];
+        const size_t cnt = cut[sgi + 1] - cut[sgi];
+        int rc = plan_forward(g, cnt, n, fo, fwd[sgi]);
+        if (!rc) rc = plan_adjoint(g, cnt, pidx ? pidx + cut[sgi] : nullptr, n, bo, bwd[sgi]);
         if (rc) return rc;
         for (int32_t p : bwd[sgi].grad_params)
             if (p < 0 || (size_t)p >= nparams) return fail(QK_ERR_ARG, "parameter %d >= %zu", p, nparams);

@@ -1,0 +1,1121 @@
+// Planner of factored pass programs (host).
+//
+// A one-qubit unitary is a scalar times diag(1, p) R diag(1, l): two phases
+// and a real rotation.  Divided by its cosine the rotation needs one
+// multiply-add a component (x' = x - t y, y' = t x + y), so
+// the unitary costs 2 (rotation) + 2 a phase multiply-adds an amplitude, where
+// the dense 2x2 of the general programs costs 8.  What is divided out is one
+// scalar for the whole state, multiplied back at the end of the plan.  Three
+// more rules shorten the programs:
+// - a left phase commutes with diagonal gates and CX controls and moves into
+//   the right phase of the next one-qubit unitary on its qubit;
+// - a two-qubit phase waits for the next one-qubit unitary on one of its
+//   qubits and then is a factor of that unitary's right phase, chosen by the
+//   other qubit's bit (one multiply a thread instead of one for half of its
+//   amplitudes), unless both qubits are register slots;
+// - CX and SWAP gates change no amplitudes: they change the labels (tile
+//   indices) a thread's amplitudes carry, and the next re-mapping writes them
+//   to their new places.
+#include <algorithm>
+#include <cmath>
+#include <complex>
+#include <cstring>
+#include <vector>
+
+#include "qk_internal.h"
+
+namespace qk {
+
+// Tile and register bits of factored passes.  complex128: 1024-amplitude
+// tiles, 16 amplitudes a thread (64 threads, eight CTAs an SM); with 2048 the
+// 28-qubit 20-layer brick circuit takes as long (65 ms) and the 28-qubit QFT
+// 25.0 against 23.9 ms, with 8 amplitudes a thread the brick takes 91 ms.
+// complex64: 4096-amplitude tiles, 32 amplitudes a thread: 75 ms on the
+// 29-qubit brick circuit against 76 ms with 2048 and 84 ms with 16 amplitudes.
+PlanOptions factored_plan_options(int dtype, int n) {
+    PlanOptions o = default_plan_options(dtype, n);
+    o.f_tile_bits = std::min(n, dtype == QK_C128 ? 10 : 12);
+    o.f_reg_bits = std::min(o.f_tile_bits, dtype == QK_C128 ? 4 : 5);
+    return o;
+}
+
+// Two-state passes, complex128 only: 512-amplitude tiles, 8 amplitudes of each
+// state a thread (24-qubit HEA of 12 layers: 25.8 ms a sweep; 26.5 with 1024,
+// 33.0 with 2048, 28.4 with 16 amplitudes).
+PlanOptions factored_adjoint_options(int dtype, int n) {
+    PlanOptions o = default_adjoint_options(dtype, n);
+    if (dtype == QK_C128) {
+        o.f_tile_bits = std::min(n, 9);
+        o.f_reg_bits = std::min(o.f_tile_bits, 3);
+    }
+    return o;
+}
+
+namespace {
+
+using cd = std::complex<double>;
+// Scalars and the factors on their way to a coefficient, which alone is
+// rounded to double (or to the state's type): with these in double the
+// 28-qubit brick circuit was 7.6e-15 off in the 2-norm.
+using cl = std::complex<long double>;
+
+cd cget(const double *m, int k) { return {m[2 * k], m[2 * k + 1]}; }
+void cset(double *m, int k, cd z) {
+    m[2 * k] = z.real();
+    m[2 * k + 1] = z.imag();
+}
+cl unit(cl z) { return z / std::abs(z); }
+cd to_double(cl z) { return {(double)z.real(), (double)z.imag()}; }
+
+// ---- gate list -> factored op list ------------------------------------------
+
+// The phases of a one-qubit gate's factors, or -1 where it is not a unitary
+// (a U1 matrix): a unitary times a scalar to a few units of rounding.
+int phases_of(const qk_gate &g, const Op &op) {
+    switch (g.kind) {
+    case QK_GATE_RY: case QK_GATE_Y: return 0;
+    case QK_GATE_H: case QK_GATE_X: return kRightPhase;   // R diag(1, -1)
+    case QK_GATE_RX: return kRightPhase | kLeftPhase;
+    default: break;
+    }
+    const cd a = cget(op.m, 0), b = cget(op.m, 1), c = cget(op.m, 2), d = cget(op.m, 3);
+    const double r0 = std::norm(a) + std::norm(b), r1 = std::norm(c) + std::norm(d);
+    const double off = std::abs(a * std::conj(c) + b * std::conj(d));
+    if (!(r0 > 1e-6 && r0 < 1e6) || !(std::fabs(r0 - r1) <= 4e-15 * r0) || !(off <= 4e-15 * r0)) return -1;
+    return kRightPhase | kLeftPhase;
+}
+
+// A two-qubit diagonal of unit entries.
+bool unit_diagonal(const Op &op) {
+    for (int k = 0; k < 4; ++k)
+        if (!(std::fabs(std::norm(cget(op.m, k)) - 1.0) <= 4e-15)) return false;
+    return true;
+}
+
+bool factorable(const qk_gate &g, Op &op) {
+    if (lower_gate(g, op)) return false;
+    switch (op.kind) {
+    case OP_DENSE1: {
+        const int ph = phases_of(g, op);
+        op.aux = ph;
+        return ph >= 0;
+    }
+    case OP_DIAG2: return unit_diagonal(op);
+    case OP_PHASE1: case OP_DIAG1: case OP_PHASE2: case OP_SWAP2: case OP_CX: case OP_PERM: return true;
+    default: return false;
+    }
+}
+
+// What the kernel has: conditions with the tile number in 32 bits, up to 512
+// threads (256 where the register amplitudes take 256 bytes), five register
+// bits for complex64 and four for complex128 (two states: complex128 with
+// three), exchange places as 16-bit offsets.
+bool sizes_fit(const PlanOptions &o, int n, int nstates) {
+    const int T = o.f_tile_bits, r = o.f_reg_bits;
+    const bool c128 = o.dtype == QK_C128;
+    if (nstates == 2 && !c128) return false;
+    return T >= 1 && T <= std::min(n, c128 ? 12 : 13) && n - T <= 31 && r >= std::min(2, T) &&
+           r <= std::min(T, nstates == 2 ? 3 : c128 ? 4 : 5) && T - r <= (((c128 ? 16 : 8) << r) * nstates >= 256 ? 8 : 9);
+}
+
+// merge_one_qubit_runs for ops that carry their phases: the product of two
+// has the outer phases, and both where a phase stands between two rotations.
+void merge_runs(std::vector<Op> &ops, int n) {
+    std::vector<long> last(n, -1);
+    std::vector<Op> out;
+    out.reserve(ops.size());
+    for (const Op &op : ops) {
+        if (one_qubit(op) && last[op.q[0]] >= 0) {
+            Op &a = out[last[op.q[0]]];
+            double x[8], y[8], z[8];
+            as_matrix(a, x);
+            as_matrix(op, y);
+            mat2_mul(y, x, z);   // op after a
+            const bool da = a.kind == OP_DENSE1, db = op.kind == OP_DENSE1;
+            if (!da && !db) {
+                a.kind = OP_DIAG1;
+                a.m[0] = z[0]; a.m[1] = z[1]; a.m[2] = z[6]; a.m[3] = z[7];
+            } else {
+                if (!da) a.aux = op.aux | kRightPhase;
+                else if (!db) a.aux |= kLeftPhase;
+                else if ((op.aux & kRightPhase) || (a.aux & kLeftPhase)) a.aux = kRightPhase | kLeftPhase;
+                else a.aux = (a.aux & kRightPhase) | (op.aux & kLeftPhase);
+                a.kind = OP_DENSE1;
+                std::memcpy(a.m, z, sizeof z);
+            }
+            continue;
+        }
+        for (int k = 0; k < op.nq; ++k) last[op.q[k]] = -1;
+        out.push_back(op);
+        if (one_qubit(op)) last[op.q[0]] = (long)out.size() - 1;
+    }
+    ops.swap(out);
+}
+
+// The scalar of an OP_K, m[6..9]: high and low parts.
+cl scalar_of(const Op &op) {
+    return {(long double)op.m[6] + op.m[8], (long double)op.m[7] + op.m[9]};
+}
+
+// OP_DENSE1 with phases aux -> OP_K.  t is the tangent of the rotation, as
+// large as it is: x - t y and t x + y round like the rotation's own rows.
+// Only a rotation by (nearly) pi has no usable tangent; its t is capped where
+// the other column's share, 1 / t, is far below a rounding.  t and the phases
+// are rounded to the state's type here and the scalar's magnitude taken from
+// the rounded values, so that their rounding does not change the norm.
+// ph: a phase the upper half still lacks; *defer: not null where the left
+// phase moves on instead, to be returned there.
+void extract(Op &op, int dtype, cl ph, cl *defer) {
+    constexpr long double cap = 0x1p64L;
+    auto rounded = [&](long double x) { return dtype == QK_C64 ? (double)(float)x : (double)x; };
+    const cl a = cget(op.m, 0), b = cl(cget(op.m, 1)) * ph, c = cget(op.m, 2), d = cl(cget(op.m, 3)) * ph;
+    const bool right = op.aux & kRightPhase, left = op.aux & kLeftPhase;
+    // M = g [[1, -t l], [p t, p l]]; from the column entry c = g p t where
+    // the tangent is large, from a = g where it is not
+    const bool large = !(std::norm(a) >= std::norm(c));
+    // the phases keep what modulus the entries give them: a matrix that is a
+    // unitary to rounding is met to rounding in all its entries
+    cl l = 1, p = 1, u = a;   // u: a multiple of g
+    long double tan;
+    if (!large) {
+        const cl q = c / a;
+        if (!left) {
+            tan = q.real();
+            if (right) l = d / a;
+        } else if (!right) {
+            tan = -(b / a).real();
+            p = d / a;
+        } else {
+            tan = std::sqrt(std::abs(q * b) / std::abs(d));
+            if (tan > 0) p = q / tan;
+            l = d / a / p;
+        }
+    } else {
+        long double k;   // 1 / tan
+        u = c;
+        if (!left) {
+            k = (a / c).real();
+            if (right) l = -b / c;
+        } else if (!right) {
+            k = -(a / b).real();
+            p = -c / b;
+            u = c / p;
+        } else {
+            const long double ra = std::abs(a);
+            u = ra > 0 ? a / ra : cl(1);
+            k = std::sqrt(ra * std::abs(d) / (std::abs(b) * std::abs(c)));
+            p = unit(c / u);
+            l = -b / u / std::abs(c);
+        }
+        if (std::signbit(k)) u = -u;   // (k may be -0)
+        tan = std::fabs(k) * cap < 1 ? std::copysign(cap, k) : 1 / k;
+    }
+    const double t = rounded(tan);
+    const cd lr(rounded(l.real()), rounded(l.imag()));
+    cd pr(rounded(p.real()), rounded(p.imag()));
+    const long double nl = std::norm(cl(lr)), np = defer ? std::norm(p) : std::norm(cl(pr)), tt = (long double)t * t;
+    const cl g = unit(u) * std::sqrt((std::norm(a) + std::norm(b) + std::norm(c) + std::norm(d)) /
+                                     (1 + tt * nl + np * (tt + nl)));
+    if (defer) *defer = p, pr = 1;
+    op.kind = OP_K;
+    std::memset(op.m, 0, sizeof op.m);
+    op.m[0] = t;
+    cset(op.m, 1, lr);
+    cset(op.m, 2, pr);
+    cset(op.m, 3, to_double(g));
+    op.m[8] = (double)(g.real() - op.m[6]);
+    op.m[9] = (double)(g.imag() - op.m[7]);
+}
+
+bool is_sign(cd f) { return f.real() == -1.0 && std::fabs(f.imag()) < 2e-16; }   // CP(pi)
+
+bool diagonal_on(const Op &op, int q) {
+    switch (op.kind) {
+    case OP_PHASE1: case OP_DIAG1: case OP_PHASE2: case OP_DIAG2: return true;
+    case OP_CX: return op.q[op.aux] == q;
+    default: return false;
+    }
+}
+
+// Merged ops -> OP_K, OP_PHASE1, OP_PHASE2, OP_CX, OP_SWAP2, OP_GRAD, OP_PERM
+// and a scalar of the whole list.  `scaled`: the list has ops with a scalar.
+void factor(std::vector<Op> &ops, int n, int dtype, cl &scale, bool &scaled) {
+    // next[i] bit k: after op i, the next op on q[k] that is not diagonal
+    // there is a one-qubit unitary, which takes in a phase on that qubit
+    std::vector<char> dense(n, 0), next(ops.size(), 0);
+    for (size_t i = ops.size(); i-- > 0;) {
+        const Op &op = ops[i];
+        for (int k = 0; k < std::min<int>(op.nq, 2); ++k) next[i] |= dense[op.q[k]] ? 1 << k : 0;
+        if (op.kind == OP_PERM) std::fill(dense.begin(), dense.end(), 0);
+        else
+            for (int k = 0; k < op.nq; ++k)
+                if (!diagonal_on(op, op.q[k])) dense[op.q[k]] = op.kind == OP_DENSE1;
+    }
+    std::vector<cl> ph(n, 1);
+    std::vector<char> has(n, 0);
+    std::vector<Op> out;
+    out.reserve(ops.size());
+    scale = 1;
+    scaled = false;
+    auto phase1 = [&](int q, cl p, bool deferred) {
+        if (deferred) {
+            ph[q] *= p;
+            has[q] = 1;
+            return;
+        }
+        Op o;
+        std::memset(&o, 0, sizeof o);
+        o.kind = OP_PHASE1;
+        o.nq = 1;
+        o.q[0] = q;
+        cset(o.m, 0, to_double(p));
+        out.push_back(o);
+    };
+    for (size_t i = 0; i < ops.size(); ++i) {
+        Op op = ops[i];
+        const int q = op.q[0];
+        switch (op.kind) {
+        case OP_DENSE1:
+            scaled = true;
+            {
+                const cl f = has[q] ? ph[q] : cl(1);
+                if (has[q]) op.aux |= kRightPhase;
+                const bool defer = (op.aux & kLeftPhase) && (next[i] & 1);
+                extract(op, dtype, f, defer ? &ph[q] : nullptr);
+                has[q] = defer;
+                if (defer) op.aux &= ~kLeftPhase;
+                else ph[q] = 1;
+            }
+            out.push_back(op);
+            break;
+        case OP_PHASE1: phase1(q, cget(op.m, 0), next[i] & 1); break;
+        case OP_DIAG1:
+            scaled = true;
+            scale *= cl(cget(op.m, 0));
+            phase1(q, cl(cget(op.m, 1)) / cl(cget(op.m, 0)), next[i] & 1);
+            break;
+        case OP_DIAG2: {
+            const cl d0 = cget(op.m, 0), d1 = cget(op.m, 1), d2 = cget(op.m, 2), d3 = cget(op.m, 3);
+            scaled = true;
+            scale *= d0;
+            phase1(op.q[0], d1 / d0, next[i] & 1);
+            phase1(op.q[1], d2 / d0, next[i] & 2);
+            op.kind = OP_PHASE2;
+            cset(op.m, 0, to_double(unit(d3 * d0 / (d1 * d2))));
+            out.push_back(op);
+            break;
+        }
+        case OP_PHASE2:
+            // CP(pi) is (-1, 1.2e-16) and runs as a change of sign.  What is
+            // dropped, exp(i e b0 b1), goes where it costs nothing: b0 b1 is
+            // (b0 + b1) / 2 - 1 / 4, b0 / 2 or 1 / 4 on average (left out, it
+            // was two thirds of the 28-qubit brick circuit's error)
+            if (is_sign(cget(op.m, 0))) {
+                const long double e = std::arg(-cl(cget(op.m, 0)));
+                const int k0 = (next[i] & 1) != 0, k1 = (next[i] & 2) != 0;
+                if (k0) phase1(op.q[0], std::polar(1.0L, e / 2), true);
+                if (k1) phase1(op.q[1], std::polar(1.0L, e / 2), true);
+                scale *= std::polar(1.0L, e * (1 - k0 - k1) / 4);
+                scaled = true;
+            }
+            out.push_back(op);
+            break;
+        default: out.push_back(op); break;
+        }
+    }
+    ops.swap(out);
+}
+
+// ---- passes -----------------------------------------------------------------
+
+bool is_work(const Op &op) { return op.kind == OP_K || op.kind == OP_GRAD; }
+
+// Tile bits an op needs (its register slot, or the labels it changes).
+int tile_bits_of(const Op &op, int (&b)[2]) {
+    switch (op.kind) {
+    case OP_K: case OP_GRAD: b[0] = op.q[0]; return 1;
+    case OP_CX: b[0] = op.q[1 - op.aux]; return 1;
+    case OP_SWAP2: b[0] = op.q[0]; b[1] = op.q[1]; return 2;
+    default: return 0;
+    }
+}
+
+struct Builder {
+    const std::vector<Op> &ops;
+    int n, T, r, L;
+    HostPlan &plan;
+    const PlanOptions &opts;
+    bool lookahead;
+    cl carry;            // scalar the stored state still lacks
+    bool scaled;
+    int grad_base = 0;
+    bool mapped = false;   // the last step is a re-mapping
+    // the TOP_LAYER being collected: its unitaries by slot
+    struct Layer {
+        int k = 0, signs = 0;   // masks
+        bool pending = false;
+        uint16_t w[8] = {0};
+        uint32_t u[8] = {0};
+        cd t[kPassMaxReg], l[kPassMaxReg];
+    } layer = Layer();
+
+    size_t amp_bytes() const { return plan.dtype == QK_C128 ? 16 : 8; }
+
+    // Shared memory a pass's program, coefficients and gradient accumulators
+    // may take besides the tile.
+    size_t budget() const {
+        const size_t tile = (amp_bytes() << T) * plan.nstates;
+        return std::min<size_t>(48u << 10, (200u << 10) - tile);
+    }
+    size_t cost(const Op &op) const {
+        const size_t c = amp_bytes();
+        switch (op.kind) {
+        case OP_K: return 40 + 3 * c;   // a share of the re-mappings included
+        case OP_GRAD: {
+            const size_t k = (int)op.m[0] == 5 ? 2 : 1;
+            return 16 + k * (2 * c + (sizeof(double) << (T - r)));
+        }
+        case OP_SWAP2: return 64;
+        default: return 24 + c;
+        }
+    }
+
+    // What the walks below look at, 16 bytes an op.
+    struct Lite {
+        uint16_t cost;
+        uint8_t nq, nb, work, perm;
+        uint8_t q[2], diag[2], b[2];   // qubits, whether diagonal there, tile bits
+    };
+    std::vector<Lite> lite = {};
+    void make_lite() {
+        lite.resize(ops.size());
+        for (size_t i = 0; i < ops.size(); ++i) {
+            const Op &op = ops[i];
+            Lite &x = lite[i];
+            std::memset(&x, 0, sizeof x);
+            x.perm = op.kind == OP_PERM;
+            if (x.perm) continue;
+            x.cost = (uint16_t)std::min<size_t>(cost(op), 65535);
+            x.nq = (uint8_t)op.nq;
+            int b[2];
+            x.nb = (uint8_t)tile_bits_of(op, b);
+            for (int k = 0; k < op.nq; ++k) x.q[k] = (uint8_t)op.q[k], x.diag[k] = diagonal_on(op, op.q[k]);
+            for (int k = 0; k < x.nb; ++k) x.b[k] = (uint8_t)b[k];
+            x.work = is_work(op) ? 4 : op.kind == OP_CX || op.kind == OP_SWAP2 ? 1 : 0;
+        }
+    }
+
+    // Walk pending ops in order; an op joins a pass on tile bits inB when no
+    // op left out before it fails to commute with it on a shared qubit, its
+    // tile bits are there (or, with grow, can be added) and the budget allows.
+    // blocked: 1 an op diagonal on the qubit was left out, 2 another op.
+    template <typename F>
+    size_t walk(const std::vector<size_t> &pending, std::vector<char> &inB, int *grow, F &&each) const {
+        char blocked[64] = {0};
+        size_t used = 256, work = 0;
+        int open = 0;   // tile bits on which work can still join
+        for (int q = 0; q < n; ++q) open += inB[q];
+        const size_t lim = budget();
+        for (size_t i : pending) {
+            const Lite &op = lite[i];
+            bool ok = !op.perm && (used == 256 || used + op.cost <= lim);
+            for (int k = 0; k < op.nq && ok; ++k) ok = blocked[op.q[k]] <= op.diag[k];
+            if (ok && op.nb) {
+                int need = 0;
+                for (int k = 0; k < op.nb; ++k) need += !inB[op.b[k]];
+                ok = need == 0 || (grow && *grow + need <= T);
+                if (ok && need)
+                    for (int k = 0; k < op.nb; ++k)
+                        if (!inB[op.b[k]]) inB[op.b[k]] = 1, ++*grow;
+            }
+            if (ok) {
+                used += op.cost;
+                work += op.work;
+            } else if (op.perm) {
+                std::memset(blocked, 2, sizeof blocked);
+                open = 0;
+            } else {
+                for (int k = 0; k < op.nq; ++k) {
+                    const char lv = op.diag[k] ? 1 : 2;
+                    open -= inB[op.q[k]] && !blocked[op.q[k]];
+                    blocked[op.q[k]] = std::max(blocked[op.q[k]], lv);
+                }
+            }
+            if (!each(i, ok)) break;
+            if (!open && !grow) break;   // counting: no more work can join
+        }
+        return work;
+    }
+
+    // Tile bits grown ahead: the first ops' bits, then one at a time the
+    // qubit of the next pending ops that lets the most work join.
+    void choose_tile(const std::vector<size_t> &pending, std::vector<char> &inB, int &nB) const {
+        auto none = [](size_t, bool) { return true; };
+        size_t base = walk(pending, inB, nullptr, none);
+        while (nB < T) {
+            std::vector<char> cand(n, 0);
+            std::vector<int> cands;
+            for (size_t j = 0, seen = 0; j < pending.size() && seen < 64; ++j) {
+                const Lite &op = lite[pending[j]];
+                seen += op.nb > 0;
+                for (int k = 0; k < op.nb; ++k)
+                    if (!inB[op.b[k]] && !cand[op.b[k]]) cand[op.b[k]] = 1, cands.push_back(op.b[k]);
+            }
+            if (cands.empty()) break;
+            int best = -1;
+            size_t bestc = base;
+            for (int q : cands) {
+                inB[q] = 1;
+                const size_t c = walk(pending, inB, nullptr, none);
+                inB[q] = 0;
+                if (c > bestc) best = q, bestc = c;
+            }
+            if (best < 0) best = cands[0];   // the earliest: a later choice may need it
+            inB[best] = 1;
+            ++nB;
+            base = bestc;
+        }
+    }
+
+    // The ops cut into passes: the ops of each and its tile bits.
+    struct Part {
+        std::vector<size_t> take;
+        std::vector<int> B;      // empty: a permutation pass, take[0]
+    };
+    std::vector<Part> parts = {};
+    void partition() {
+        make_lite();
+        std::vector<size_t> pending(ops.size()), rest;
+        for (size_t i = 0; i < ops.size(); ++i) pending[i] = i;
+        while (!pending.empty()) {
+            Part p;
+            if (lite[pending[0]].perm) {
+                p.take.push_back(pending[0]);
+                pending.erase(pending.begin());
+                parts.push_back(std::move(p));
+                continue;
+            }
+            std::vector<char> inB(n, 0);
+            int nB = 0;
+            for (int q = 0; q < std::min(n, L); ++q) inB[q] = 1, ++nB;
+            if (lookahead) choose_tile(pending, inB, nB);
+            rest.clear();
+            walk(pending, inB, &nB, [&](size_t i, bool ok) {
+                (ok ? p.take : rest).push_back(i);
+                return true;
+            });
+            defer(p.take, rest);
+            for (int q = 0; q < n && nB < T; ++q)
+                if (!inB[q]) inB[q] = 1, ++nB;
+            for (int q = 0; q < n; ++q)
+                if (inB[q]) p.B.push_back(q);
+            parts.push_back(std::move(p));
+            pending.swap(rest);
+        }
+    }
+
+    int compile_parts() {
+        size_t last = parts.size();   // the last compute pass
+        while (last && parts[last - 1].B.empty()) --last;
+        for (size_t k = 0; k < parts.size(); ++k) {
+            if (!parts[k].B.empty()) {
+                int rc = compile(parts[k].take, parts[k].B, k + 1 == last);
+                if (rc) return rc;
+                continue;
+            }
+            flush();
+            HostPlan one;
+            int rc = build_perm_plan(ops[parts[k].take[0]], n, opts, one);
+            if (rc) return rc;
+            plan.passes.push_back(one.passes[0]);
+            plan.ngates += 1;
+        }
+        return QK_OK;
+    }
+
+    // Ops of the pass that no unitary or gradient of it follows wait for a
+    // later pass when one does there: a phase then joins that unitary, a CX
+    // the re-mapping before it.
+    void defer(std::vector<size_t> &take, std::vector<size_t> &rest) const {
+        std::vector<char> touched(n, 0);   // by ops of rest: 1 diagonal only, 2 else
+        bool any = false;
+        for (size_t i : rest)
+            if (ops[i].kind != OP_PERM)
+                for (int k = 0; k < ops[i].nq; ++k)
+                    touched[ops[i].q[k]] = std::max<char>(touched[ops[i].q[k]], diagonal_on(ops[i], ops[i].q[k]) ? 1 : 2);
+        std::vector<char> keep(take.size(), 0), need(n, 0);   // need: by kept ops, as touched
+        for (size_t k = take.size(); k-- > 0;) {
+            const Op &op = ops[take[k]];
+            bool kp = is_work(op), later = false;
+            for (int j = 0; j < op.nq; ++j) {
+                const bool dg = diagonal_on(op, op.q[j]);
+                kp = kp || need[op.q[j]] > (dg ? 1 : 0);
+                later = later || touched[op.q[j]] > (dg ? 1 : 0);
+            }
+            kp = kp || !later;
+            keep[k] = kp;
+            any = any || kp;
+            if (kp)
+                for (int j = 0; j < op.nq; ++j)
+                    need[op.q[j]] = std::max<char>(need[op.q[j]], diagonal_on(op, op.q[j]) ? 1 : 2);
+        }
+        if (!any) return;
+        std::vector<size_t> t2;
+        for (size_t k = 0; k < take.size(); ++k)
+            (keep[k] ? t2 : rest).push_back(take[k]);
+        take.swap(t2);
+        std::sort(rest.begin(), rest.end());
+    }
+
+    // ---- one pass ----
+    struct Pass {
+        std::vector<size_t> idx;
+        std::vector<int> work;       // positions of unitaries and gradients not yet done
+        std::vector<std::vector<int>> preds;
+        std::vector<char> done;
+        std::vector<int> local, Q;   // state bit -> tile bit or -1; slots (tile bits, ascending)
+        std::vector<int> outer;      // state bit outside the tile -> bit of the tile number
+        std::vector<char> dirty;     // per state bit: 1 CX control, 2 label changed since the re-mapping
+        size_t left = 0, work_left = 0;
+    };
+
+    int slot(const Pass &P, int q) const {
+        const int b = P.local[q];
+        if (b < 0) return -1;
+        const auto it = std::find(P.Q.begin(), P.Q.end(), b);
+        return it == P.Q.end() ? -1 : (int)(it - P.Q.begin());
+    }
+    bool is_phase(const Op &op) const { return op.kind == OP_PHASE1 || op.kind == OP_PHASE2; }
+    bool is_phase(const Lite &op) const { return !op.nb && !op.perm; }
+
+    // Undone predecessors of op k that are phases which can run now; false
+    // when another predecessor is undone.
+    bool pending_phases(const Pass &P, const std::vector<char> &done, int k, std::vector<int> *out) const {
+        if (out) out->clear();
+        for (int p : P.preds[k]) {
+            if (done[p]) continue;
+            const Lite &o = lite[P.idx[p]];
+            if (!is_phase(o)) return false;
+            for (int j = 0; j < o.nq; ++j)
+                if (P.dirty[o.q[j]] > 1) return false;
+            for (int pp : P.preds[p])
+                if (!done[pp]) return false;
+            if (out) out->push_back(p);
+        }
+        return true;
+    }
+
+    // Run (emit) or count the work that can run under slots P.Q.
+    size_t run_work(Pass &P, bool emit) {
+        std::vector<char> copy;
+        if (!emit) copy = P.done;
+        std::vector<char> &done = emit ? P.done : copy;
+        std::vector<int> ph;
+        size_t cnt = 0;
+        bool trim = false;
+        for (bool progress = true; progress;) {
+            progress = false;
+            for (int k : P.work) {
+                const int q = lite[P.idx[k]].q[0];
+                if (done[k] || slot(P, q) < 0 || P.dirty[q]) continue;
+                if (!pending_phases(P, done, k, &ph)) continue;
+                const Op &op = ops[P.idx[k]];
+                for (int p : ph) done[p] = 1;
+                done[k] = 1;
+                ++cnt;
+                progress = true;
+                if (!emit) continue;
+                trim = true;
+                P.left -= 1 + ph.size();
+                --P.work_left;
+                if (op.kind == OP_K) emit_k(P, op, ph);
+                else {
+                    for (int p : ph) emit_phase(P, ops[P.idx[p]]);
+                    emit_grad(P, op);
+                }
+            }
+        }
+        if (trim)
+            P.work.erase(std::remove_if(P.work.begin(), P.work.end(), [&](int k) { return P.done[k] != 0; }), P.work.end());
+        return cnt;
+    }
+
+    // CX and SWAP labels (and, once no work is left, the remaining phases).
+    bool run_labels(Pass &P) {
+        bool changed = false;
+        std::vector<int> ph;
+        for (bool progress = true; progress;) {
+            progress = false;
+            for (size_t k = 0; k < P.idx.size(); ++k) {
+                const Op &op = ops[P.idx[k]];
+                if (P.done[k] || is_work(op)) continue;
+                if (is_phase(op)) {
+                    if (P.work_left) continue;
+                    bool ok = true;
+                    for (int j = 0; j < op.nq; ++j) ok = ok && P.dirty[op.q[j]] < 2;
+                    for (int p : P.preds[k]) ok = ok && P.done[p];
+                    if (!ok) continue;
+                    emit_phase(P, op);
+                } else {
+                    if (!pending_phases(P, P.done, (int)k, &ph)) continue;
+                    for (int p : ph) {
+                        emit_phase(P, ops[P.idx[p]]);
+                        P.done[p] = 1;
+                        --P.left;
+                    }
+                    changed = true;
+                    if (op.kind == OP_CX) {
+                        label(P, op.q[1 - op.aux], op.q[op.aux]);
+                        P.dirty[op.q[op.aux]] = std::max<char>(P.dirty[op.q[op.aux]], 1);
+                        P.dirty[op.q[1 - op.aux]] = 2;
+                    } else {
+                        label(P, op.q[0], op.q[1]);
+                        label(P, op.q[1], op.q[0]);
+                        label(P, op.q[0], op.q[1]);
+                        P.dirty[op.q[0]] = P.dirty[op.q[1]] = 2;
+                    }
+                }
+                P.done[k] = 1;
+                --P.left;
+                progress = true;
+            }
+        }
+        return changed;
+    }
+
+    // 16 bytes that belong to the step before.
+    void word(const void *p, size_t bytes) {
+        TOp x;
+        std::memset(&x, 0, sizeof x);
+        std::memcpy(&x, p, bytes);
+        plan.ops.push_back(x);
+    }
+    // The collected layer as a step.
+    void flush() {
+        if (!layer.k && !layer.signs) return;
+        const Layer y = layer;
+        layer = Layer();
+        bool words = false;
+        for (int s = 0; s < kPassMaxReg; ++s) words = words || y.u[s] || y.w[s];
+        TOp &t = step(TOP_LAYER);
+        t.a = (uint8_t)y.k;
+        t.b = (uint8_t)((words ? kLayerWords : 0) | (y.signs ? kLayerSigns : 0) | (y.pending ? kLayerPending : 0));
+        t.bits[0] = (uint8_t)y.signs;
+        t.bits[1] = (uint8_t)(y.signs >> 8);
+        if (words) {
+            t.nbits = 2;   // u[0..3]; u[4] and w[0..4]
+            word(y.u, 16);
+            unsigned char b[16] = {0};
+            std::memcpy(b, y.u + 4, 4);
+            std::memcpy(b + 4, y.w, 10);
+            word(b, 16);
+        }
+        for (int s = 0; s < kPassMaxReg; ++s) {
+            if (!((y.k >> s) & 1)) continue;
+            push(y.t[s]);
+            push(y.l[s]);
+        }
+    }
+    TOp &step(uint8_t kind) {
+        flush();
+        // steps under one re-mapping count as one program operation
+        if (kind == TOP_REMAP) ++plan.nremaps;
+        else if (mapped) ++plan.nbodies;
+        mapped = kind == TOP_REMAP;
+        TOp t;
+        std::memset(&t, 0, sizeof t);
+        t.kind = kind;
+        t.coef = (uint32_t)(plan.coef.size() / 2);
+        plan.ops.push_back(t);
+        return plan.ops.back();
+    }
+    void push(cd z) {
+        plan.coef.push_back(z.real());
+        plan.coef.push_back(z.imag());
+    }
+    uint8_t code(const Pass &P, int q) const {
+        return P.local[q] >= 0 ? (uint8_t)P.local[q] : (uint8_t)(kOuterFlag | q);
+    }
+    void label(const Pass &P, int target, int control) {
+        TOp &t = step(TOP_LCX);
+        t.a = (uint8_t)P.local[target];
+        t.b = code(P, control);
+    }
+    void remap(Pass &P, const std::vector<int> &Q, bool dirty) {
+        P.Q = Q;
+        std::sort(P.Q.begin(), P.Q.end());
+        std::fill(P.dirty.begin(), P.dirty.end(), 0);
+        TOp &t = step(TOP_REMAP);
+        t.nbits = 1;
+        t.b = dirty;
+        uint16_t off[kPassMaxReg] = {0};
+        for (int s = 0; s < r; ++s) {
+            t.bits[s] = (uint8_t)P.Q[s];
+            off[s] = (uint16_t)(tile_swizzle(1u << P.Q[s], plan.dtype == QK_C128) * amp_bytes());
+        }
+        word(off, sizeof off);
+    }
+    void emit_phase(Pass &P, const Op &op) {
+        const int sa = slot(P, op.q[0]), sb = op.nq > 1 ? slot(P, op.q[1]) : -1;
+        if (sa >= 0 && sb >= 0 && is_sign(cget(op.m, 0))) {
+            // the layer's signs come before its unitaries
+            if (((layer.k >> sa) | (layer.k >> sb)) & 1) flush();
+            layer.signs ^= 1 << slot_pair(std::min(sa, sb), std::max(sa, sb));
+            return;
+        }
+        if (sa >= 0 && sb >= 0) {
+            step((uint8_t)(TOP_PH2 + slot_pair(std::min(sa, sb), std::max(sa, sb))));
+        } else {
+            TOp &t = step(TOP_PHASE);
+            t.a = code(P, op.q[0]);
+            t.b = op.nq > 1 ? code(P, op.q[1]) : kNoQubit;
+            t.bits[0] = sa >= 0 ? (uint8_t)sa : kNoSlot;
+            t.bits[1] = sb >= 0 ? (uint8_t)sb : kNoSlot;
+        }
+        push(cget(op.m, 0));
+    }
+    void emit_k(Pass &P, const Op &op, const std::vector<int> &ph) {
+        // conditions: phases whose other qubit is the same for all of a
+        // thread's amplitudes; those between two slots run as steps before
+        std::vector<std::pair<uint8_t, cd>> cond;
+        for (int p : ph) {
+            const Op &o = ops[P.idx[p]];
+            const int x = o.nq == 1 ? -1 : o.q[0] == op.q[0] ? o.q[1] : o.q[0];
+            if (x >= 0 && slot(P, x) >= 0) {
+                emit_phase(P, o);
+                continue;
+            }
+            const cd f = cget(o.m, 0);
+            cond.push_back({x < 0 ? kNoQubit : (uint8_t)(code(P, x) | (is_sign(f) ? kSignFlag : 0)), f});
+        }
+        // amplitudes grow by 1 / |scalar|; before their magnitude leaves a
+        // quarter of the type's exponent range it is set back
+        const double range = plan.dtype == QK_C128 ? 0x1p-200 : 0x1p-60;
+        if (std::abs(carry * scalar_of(op)) < range) {
+            const double f = rounded((double)std::abs(carry));
+            step(TOP_SCALE);
+            push(f);
+            carry /= f;
+        }
+        carry *= scalar_of(op);
+        bool simple = true;   // conditions that only change the sign
+        for (const auto &c : cond) simple = simple && c.first != kNoQubit && (c.first & kSignFlag);
+        const int s = slot(P, op.q[0]);
+        if (!simple) {
+            if (op.aux & kRightPhase) cond.push_back({kNoQubit, cget(op.m, 1)});   // part of the pending factor
+            for (size_t c0 = 0; c0 < cond.size(); c0 += 8) {
+                TOp &t = step(TOP_LAM);
+                for (size_t i = c0; i < std::min(c0 + 8, cond.size()); ++i) t.bits[t.nbits++] = cond[i].first;
+                for (size_t i = c0; i < std::min(c0 + 8, cond.size()); ++i)
+                    if (cond[i].first == kNoQubit || !(cond[i].first & kSignFlag)) push(cond[i].second);
+            }
+        } else if ((layer.k >> s) & 1) {
+            flush();
+        }
+        layer.k |= 1 << s;
+        layer.t[s] = op.m[0];
+        layer.l[s] = cget(op.m, 1);
+        if (!simple) {   // the pending factor is for this unitary alone
+            layer.pending = true;
+            flush();
+        } else {
+            for (const auto &c : cond) {
+                if (c.first & kOuterFlag) layer.u[s] ^= 1u << P.outer[c.first & 0x3F];
+                else layer.w[s] ^= (uint16_t)(1u << (c.first & 0x3F));
+            }
+        }
+        if (op.aux & kLeftPhase) {
+            TOp &t = step(TOP_PHASE);
+            t.a = code(P, op.q[0]);
+            t.b = kNoQubit;
+            t.bits[0] = (uint8_t)s;
+            t.bits[1] = kNoSlot;
+            push(cget(op.m, 2));
+        }
+    }
+    double rounded(double x) const { return plan.dtype == QK_C64 ? (double)(float)x : x; }
+    void emit_grad(Pass &P, const Op &op) {
+        // both states lack the factor carry: the sums grow by its square
+        const double f = (double)std::norm(carry);
+        const int gen = (int)op.m[0];
+        TOp &t = step(TOP_GRAD);
+        t.a = (uint8_t)slot(P, op.q[0]);
+        t.b = gen == 5 ? 5 : 4;
+        auto param_slot = [&](int32_t p) {
+            int k = grad_base;
+            while (k < (int)plan.grad_params.size() && plan.grad_params[k] != p) ++k;
+            if (k == (int)plan.grad_params.size()) plan.grad_params.push_back(p);
+            return k - grad_base;
+        };
+        const int k1 = param_slot(op.aux);
+        t.bits[0] = (uint8_t)(k1 & 0xFF);
+        t.bits[1] = (uint8_t)(k1 >> 8);
+        if (gen == 5) {
+            const int k2 = param_slot((int32_t)op.m[8]);
+            t.bits[2] = (uint8_t)(k2 & 0xFF);
+            t.bits[3] = (uint8_t)(k2 >> 8);
+        }
+        const double a = gen == 1 ? 1 : gen >= 4 ? op.m[2] : 0, b = gen == 2 ? 1 : gen >= 4 ? op.m[3] : 0,
+                     c = gen == 3 ? 1 : gen >= 4 ? op.m[4] : 0;
+        push({f * a, f * b});
+        push({f * c, 0});
+        if (gen == 5) {
+            push({f * op.m[5], f * op.m[6]});
+            push({f * op.m[7], 0});
+        }
+    }
+
+    // Slots for the next re-mapping: grown by the tile bit that lets the most
+    // work run (ties: the bit of the earliest work), then the highest bits.
+    // Under the first mapping the tile is loaded, so its slots leave the
+    // lowest L bits to the threads (runs of contiguous amplitudes).
+    std::vector<int> choose_slots(Pass &P, bool first, int lo) {
+        std::vector<int> cand, Q;
+        for (int k : P.work) {
+            const int b = P.local[lite[P.idx[k]].q[0]];
+            if ((!first || b >= lo) && std::find(cand.begin(), cand.end(), b) == cand.end()) cand.push_back(b);
+        }
+        size_t base = 0;
+        while ((int)Q.size() < r && !cand.empty()) {
+            int best = -1;
+            size_t bestc = base;
+            for (size_t i = 0; i < cand.size(); ++i) {
+                P.Q = Q;
+                P.Q.push_back(cand[i]);
+                const size_t c = run_work(P, false);
+                if (c > bestc) best = (int)i, bestc = c;
+            }
+            if (best < 0) best = 0;
+            Q.push_back(cand[best]);
+            cand.erase(cand.begin() + best);
+            base = bestc;
+        }
+        fill_high(Q);
+        return Q;
+    }
+    void fill_high(std::vector<int> &Q) const {
+        for (int b = T - 1; b >= 0 && (int)Q.size() < r; --b)
+            if (std::find(Q.begin(), Q.end(), b) == Q.end()) Q.push_back(b);
+    }
+
+    int compile(const std::vector<size_t> &idx, const std::vector<int> &B, bool last_pass) {
+        PassDesc d;
+        std::memset(&d, 0, sizeof d);
+        d.form = 1;
+        d.T = (int)B.size();
+        for (int k = 0; k < d.T; ++k) d.bpos[k] = B[k];
+        while (d.L < d.T && d.bpos[d.L] == d.L) ++d.L;
+        Pass P;
+        P.idx = idx;
+        P.local.assign(n, -1);
+        for (int k = 0; k < d.T; ++k) P.local[B[k]] = k;
+        P.outer.assign(n, -1);
+        for (int q = 0, k = 0; q < n; ++q)
+            if (P.local[q] < 0) P.outer[q] = k++;
+        P.dirty.assign(n, 0);
+        P.done.assign(idx.size(), 0);
+        P.preds.resize(idx.size());
+        P.left = idx.size();
+        // predecessors: ops that share a qubit and are not both diagonal on it
+        std::vector<int> lastn(n, -1);
+        std::vector<std::vector<int>> diags(n);
+        for (size_t k = 0; k < idx.size(); ++k) {
+            const Op &op = ops[idx[k]];
+            if (is_work(op)) P.work.push_back((int)k);
+            P.work_left += is_work(op);
+            for (int j = 0; j < op.nq; ++j) {
+                const int q = op.q[j];
+                if (lastn[q] >= 0) P.preds[k].push_back(lastn[q]);
+                if (diagonal_on(op, q)) {
+                    diags[q].push_back((int)k);
+                } else {
+                    P.preds[k].insert(P.preds[k].end(), diags[q].begin(), diags[q].end());
+                    diags[q].clear();
+                    lastn[q] = (int)k;
+                }
+            }
+            std::sort(P.preds[k].begin(), P.preds[k].end());
+            P.preds[k].erase(std::unique(P.preds[k].begin(), P.preds[k].end()), P.preds[k].end());
+        }
+        d.prog0 = (int)plan.ops.size();
+        d.coef0 = (int)(plan.coef.size() / 2);
+        d.grad0 = grad_base = (int)plan.grad_params.size();
+        // slots of the first and last mapping stay off the lowest bits
+        const int lo = T - L >= r ? L : 0;
+        bool dirty = false;   // a label step has run since the last re-mapping
+        remap(P, choose_slots(P, true, lo), false);
+        for (bool first = true;; first = false) {
+            const size_t before = P.left;
+            run_work(P, true);
+            dirty = run_labels(P) || dirty;
+            if (!P.left) break;
+            if (!first && P.left == before) return fail(QK_ERR_ARG, "planner: a pass makes no progress");
+            remap(P, choose_slots(P, false, lo), dirty);
+            dirty = false;
+        }
+        flush();
+        if (dirty || (!P.Q.empty() && P.Q[0] < lo)) {
+            std::vector<int> Q;
+            fill_high(Q);
+            remap(P, Q, dirty);
+        }
+        if (scaled && last_pass) {
+            TOp &t = step(TOP_SCALE);
+            t.b = 1;
+            push({(double)carry.real(), (double)carry.imag()});
+            carry = 1;
+        }
+        d.nprog = (int)plan.ops.size() - d.prog0;
+        d.ncoef = (int)(plan.coef.size() / 2) - d.coef0;
+        d.ngrad = (int)plan.grad_params.size() - d.grad0;
+        for (int i = 0; i < d.nprog; ++i) {
+            TOp &t = plan.ops[d.prog0 + i];
+            if (t.kind == TOP_REMAP) d.last = i;
+            else t.coef -= (uint32_t)d.coef0;
+            if (t.kind == TOP_REMAP || t.kind == TOP_LAYER) i += t.nbits;   // the words after it
+        }
+        for (int s = 0; s < r; ++s) {
+            d.fpos[s] = B[plan.ops[d.prog0].bits[s]];
+            d.lpos[s] = B[plan.ops[d.prog0 + d.last].bits[s]];
+        }
+        plan.passes.push_back(d);
+        plan.ngates += idx.size();
+        return QK_OK;
+    }
+};
+
+// The candidates of a plan: op lists, each in both orders and with both ways
+// to choose tiles.  All are cut into passes; of those with the fewest passes
+// the first and the last are compiled, the one with fewer re-mappings kept.
+int build_best(const std::vector<std::vector<Op>> &lists, const std::vector<cl> &scale, const std::vector<char> &scaled,
+               int n, const PlanOptions &o, int nstates, HostPlan &plan) {
+    PlanOptions fo = o;
+    fo.tile_bits = o.f_tile_bits;
+    const int L = pass_low_bits(fo, n);
+    struct Candidate {
+        size_t list = 0;
+        std::vector<Op> ops;
+        std::vector<Builder::Part> parts;
+    } first, last;
+    HostPlan empty;
+    empty.n = n;
+    empty.dtype = o.dtype;
+    empty.T = o.f_tile_bits;
+    empty.r = o.f_reg_bits;
+    empty.nstates = nstates;
+    bool have = false, two = false;
+    for (size_t list = 0; list < lists.size(); ++list)
+        for (int variant = 0; variant < 4; ++variant) {
+            Candidate c;
+            c.list = list;
+            c.ops = lists[list];
+            if (variant % 2) asap_order(c.ops, n);
+            Builder b{c.ops, n, o.f_tile_bits, o.f_reg_bits, L, empty, o, variant >= 2, scale[list], scaled[list] != 0};
+            b.partition();
+            if (have && b.parts.size() > first.parts.size()) continue;
+            c.parts.swap(b.parts);
+            two = have && c.parts.size() == first.parts.size();
+            std::swap(two ? last : first, c);
+            have = true;
+        }
+    for (Candidate *c : {&first, &last}) {
+        if (c == &last && !two) break;
+        HostPlan hp = empty;
+        Builder b{c->ops, n, o.f_tile_bits, o.f_reg_bits, L, hp, o, false, scale[c->list], scaled[c->list] != 0};
+        b.make_lite();
+        b.parts.swap(c->parts);
+        int rc = b.compile_parts();
+        if (rc) return rc;
+        if (c == &first || hp.nremaps < plan.nremaps) plan = std::move(hp);
+    }
+    return QK_OK;
+}
+
+}  // namespace
+
+bool plan_is_factored(const qk_gate *gates, size_t ng, int n, const PlanOptions &o, int nstates) {
+    if (!sizes_fit(o, n, nstates)) return false;
+    for (size_t i = 0; i < ng; ++i) {
+        Op op;
+        if (!factorable(gates[i], op)) return false;
+        for (int k = 0; k < op.nq; ++k)
+            if (op.q[k] < 0 || op.q[k] >= n) return false;
+    }
+    return true;
+}
+
+int plan_forward(const qk_gate *gates, size_t ng, int n, const PlanOptions &o, HostPlan &plan) {
+    int rc = check_options(o, n);
+    if (rc) return rc;
+    if (!plan_is_factored(gates, ng, n, o, 1)) return build_plan(gates, ng, n, o, plan);
+    std::vector<Op> lowered(ng);
+    bool swaps = false;
+    for (size_t i = 0; i < ng; ++i) {
+        factorable(gates[i], lowered[i]);
+        swaps = swaps || (lowered[i].kind == OP_SWAP2 && lowered[i].aux != 1);
+    }
+    // SWAP gates as label steps, or as renamings too
+    std::vector<std::vector<Op>> lists;
+    std::vector<cl> scale;
+    std::vector<char> scaled;
+    for (int rename = 0; rename <= (swaps ? 1 : 0); ++rename) {
+        std::vector<Op> ops = lowered;
+        relabel_perms(ops, n, pass_low_bits(o, n), perm_tile_bits(o.dtype), 6, rename);
+        merge_runs(ops, n);
+        cl f;
+        bool has;
+        factor(ops, n, o.dtype, f, has);
+        lists.push_back(std::move(ops));
+        scale.push_back(f);
+        scaled.push_back(has);
+    }
+    return build_best(lists, scale, scaled, n, o, 1, plan);
+}
+
+int plan_adjoint(const qk_gate *gates, size_t ng, const int32_t *pidx, int n, const PlanOptions &o, HostPlan &plan) {
+    int rc = check_options(o, n);
+    if (rc) return rc;
+    if (!plan_is_factored(gates, ng, n, o, 2)) return build_adjoint_plan(gates, ng, pidx, n, o, plan);
+    std::vector<Op> ops;
+    ops.reserve(2 * ng);
+    for (size_t i = ng; i-- > 0;) {
+        Op op;
+        factorable(gates[i], op);
+        if (pidx && pidx[i] >= 0) {
+            const int gen = gates[i].kind == QK_GATE_RX ? 1 : gates[i].kind == QK_GATE_RY ? 2 : gates[i].kind == QK_GATE_RZ ? 3 : 0;
+            if (!gen) return fail(QK_ERR_UNSUPPORTED, "gate %zu: only RX, RY, RZ are trainable", i);
+            Op g;
+            std::memset(&g, 0, sizeof g);
+            g.kind = OP_GRAD;
+            g.nq = 1;
+            g.q[0] = op.q[0];
+            g.m[0] = gen;
+            g.aux = pidx[i];
+            ops.push_back(g);
+        }
+        invert_op(op);   // the inverse of each single gate has the gate's phases
+        ops.push_back(op);
+    }
+    hoist_gradients(ops, n);
+    merge_runs(ops, n);
+    pair_gradients(ops);
+    cl scale;
+    bool scaled;
+    factor(ops, n, o.dtype, scale, scaled);
+    return build_best({ops}, {scale}, {scaled}, n, o, 2, plan);
+}
+
+int build_group_plan(const qk_gate *gates, const int32_t *sizes, size_t ngroups, int n, const PlanOptions &o,
+                     HostPlan &plan) {
+    size_t ng = 0;
+    for (size_t g = 0; g < ngroups; ++g) {
+        if (sizes[g] < 0) return fail(QK_ERR_ARG, "group %zu has negative size", g);
+        ng += (size_t)sizes[g];
+    }
+    // The groups bound nothing here: a tile can hold any qubits, and VSWAP
+    // groups become renamings, so the gates of all groups are planned as one
+    // gate list.
+    return plan_forward(gates, ng, n, o, plan);
+}
+
+}  // namespace qk

@@ -25,7 +25,11 @@ enum OpKind : int32_t {
     OP_GRAD = 8,    // adjoint sweep: grad[aux] += Im <lambda|G|psi>, G on q[0] = X/Y/Z by m[0] = 1/2/3
     OP_CX = 9,      // flip bit q[1 - aux] where bit q[aux] is set (a U2 that is exactly a CNOT)
     OP_CDENSE1 = 10,  // 2x2 on q[0]: m[0..7] where bit q[1] is 0, m[8..15] where it is 1 (planner-made)
+    OP_K = 11,  // factored one-qubit unitary on q[0], without its scalar (planner-made, qk_factor.cpp):
+                // right phase m[2..3] on the upper half, then x' = x - t y, y' = t x + y, t = m[0], then
+                // left phase m[4..5]; scalar m[6..7]; aux = kRightPhase | kLeftPhase
 };
+constexpr int kRightPhase = 1, kLeftPhase = 2;
 
 struct Op {
     int32_t kind;
@@ -87,7 +91,30 @@ enum TOpKind : uint8_t {
     TOP_CG1 = 7,    // dense 2x2 on slot a: coef[0..3] or coef[4..7] by qubit code b (not a register slot)
     TOP_R1 = 8,     // real 2x2 on slot a: coef[0] = (m00, m01), coef[1] = (m10, m11)
     TOP_R2 = 9,     // real 4x4 on slots a < b (index bit0 = a): coef[2 r + h] = (m[r][2h], m[r][2h + 1])
+
+    // Steps of factored programs (PassDesc.form = 1, qk_factor.cpp); nbits of a TOP_REMAP or TOP_LAYER
+    // counts the 16-byte words that follow it and are no steps themselves.  Their
+    // slots are ascending in the tile bits, the first op is the TOP_REMAP the
+    // tile is loaded under, and the last TOP_REMAP the one it is stored under.
+    // TOP_REMAP: the slots in bits, b = 1 if a TOP_LCX ran since the last one; the next word holds five
+    // 16-bit values, the exchange-buffer byte offset of each slot's tile bit.
+    // TOP_LAYER: factored one-qubit unitaries on several slots.  First, with kLayerSigns in b,
+    // amplitudes whose slots x and y are both 1 change sign for each pair x < y in the mask bits[0..1].
+    // Then for each slot s in a, ascending, a unitary with coefficients t and right phase: the slot's
+    // upper half y takes the right phase (kLayerPending: the pending factor instead) and, with
+    // kLayerWords, a sign, the parity of (tile label & w[s]) and (tile number & u[s]); the next two
+    // words hold u, five 32-bit values, and w, five 16-bit values.  Then x' = x - t y, y' = t x + y
+    TOP_LAYER = 14,
+    TOP_LCX = 15,   // label step: tile bit a ^= qubit code b (a CX whose swap the next TOP_REMAP performs)
+    TOP_PH2 = 16,   // 16 + slot_pair(a, b): amplitude *= coef[0] where slots a and b are 1
+    TOP_LAM = 28,   // pending factor of the next TOP_LAYER: for each of the nbits <= 8 condition codes
+                    // in bits whose qubit is 1 times the next coef, or -1 for a code with kSignFlag
+    TOP_SCALE = 29, // amplitude *= coef[0] (b = 1: complex, 0: its real part)
 };
+constexpr uint8_t kLayerWords = 0x20, kLayerSigns = 0x40, kLayerPending = 0x80;   // TOP_LAYER, high half of b
+constexpr uint8_t kSignFlag = 0x40;   // condition codes of factored steps: the factor is -1
+// index of the slot pair a < b among 0..9 (five slots)
+constexpr int slot_pair(int a, int b) { return b * (b - 1) / 2 + a; }
 // The kernel instance for passes marked xops carries factors that are the
 // same for all of a thread's amplitudes (TOP_DIAG / TOP_PHASE on qubits
 // outside the register slots) as one pending scalar, applied before the
@@ -105,6 +132,14 @@ constexpr bool pending_scalar_ok(int amp_bytes, int reg_amps, int nstates) {
 constexpr uint8_t kOuterFlag = 0x80;
 constexpr uint8_t kNoQubit = 0xFF;
 
+// Place of tile element j in a shared-memory tile: the low index bits XORed
+// with folds of the higher ones, so that a warp's lanes, which differ in
+// three (complex128) or four (complex64) consecutive thread bits wherever the
+// register slots sit, address distinct banks.
+constexpr uint32_t tile_swizzle(uint32_t j, bool c128) {
+    return c128 ? j ^ (((j >> 3) ^ (j >> 6) ^ (j >> 9) ^ (j >> 12)) & 7u) : j ^ (((j >> 4) ^ (j >> 8) ^ (j >> 12)) & 15u);
+}
+
 struct TOp {
     uint8_t kind;
     uint8_t a, b;
@@ -113,6 +148,7 @@ struct TOp {
     uint32_t coef;
 };
 static_assert(sizeof(TOp) == 16, "TOp must stay 16 bytes");
+static_assert(offsetof(TOp, bits) == 4 && offsetof(TOp, coef) == 12, "step words follow the fields");
 constexpr uint8_t kNoSlot = 0xFF;   // TOp.bits[k] of a condition qubit held in no register slot
 
 struct PassDesc {
@@ -127,6 +163,9 @@ struct PassDesc {
     int32_t perm_a[6], perm_b[6]; // tile-local bit pairs swapped on store (perm passes)
     int32_t xops;                 // 1: the program has real or diagonal ops (TOP_R1, TOP_R2, TOP_DIAG,
                                   // TOP_PHASE), run by the kernel instance that specialises them
+    int32_t form;                 // 1: a factored program (k_fpass)
+    int32_t last;                 // factored: index of the program's last TOP_REMAP
+    int32_t fpos[kPassMaxReg], lpos[kPassMaxReg];  // factored: state bits of the first / last mapping's slots
 };
 
 // Host plan: passes + programs + complex coefficient pool (FP64).
@@ -140,6 +179,10 @@ struct HostPlan {
     std::vector<int32_t> grad_params;  // parameter index of each pass's gradient slots
     int nstates = 1;           // 2: adjoint passes over (psi, lambda)
     size_t nremaps = 0, ngates = 0;
+    // factored programs: program operations, a re-mapping and the steps that
+    // run under it counting one each
+    size_t nbodies = 0;
+    size_t program_ops() const { return nbodies ? nremaps + nbodies : ops.size(); }
 };
 
 struct PlanOptions {
@@ -148,8 +191,23 @@ struct PlanOptions {
     int reg_bits;    // r
     int plain_ops = 0;    // 1: no TOP_R1 / TOP_R2 (real ops as TOP_G1 / TOP_G2) and no pass marked
                           // xops (plans of the batched kernel, which has one instance)
+    // plan_forward / plan_adjoint: tile and register bits of factored programs,
+    // which are made where they can be (0: general programs only)
+    int f_tile_bits = 0, f_reg_bits = 0;
 };
 
+// The fused plan of a flat gate list / of a backward sweep as the engine runs
+// it: factored programs (qk_factor.cpp) where every one-qubit gate is a
+// unitary and every two-qubit gate diagonal, a CX or a SWAP, and the kernel has
+// the tile shape (complex128 only for backward sweeps); else the general programs of build_plan /
+// build_adjoint_plan.
+int plan_forward(const qk_gate *gates, size_t ng, int n, const PlanOptions &o, HostPlan &plan);
+int plan_adjoint(const qk_gate *gates, size_t ng, const int32_t *pidx, int n, const PlanOptions &o, HostPlan &plan);
+// Whether a plan of these options and gates is factored.
+bool plan_is_factored(const qk_gate *gates, size_t ng, int n, const PlanOptions &o, int nstates);
+int check_options(const PlanOptions &o, int n);
+int pass_low_bits(const PlanOptions &o, int n);
+int perm_tile_bits(int dtype);
 // Build a fused plan for a flat gate list (greedy tile-bit choice).
 int build_plan(const qk_gate *gates, size_t ng, int n, const PlanOptions &o, HostPlan &plan);
 // One permutation pass (an OP_PERM of 1 to 6 bit pairs), with no program.
@@ -170,6 +228,9 @@ void relabel_perms(std::vector<Op> &ops, int n, int L, int max_bits, int max_pai
 int build_group_plan(const qk_gate *gates, const int32_t *sizes, size_t ngroups, int n, const PlanOptions &o,
                      HostPlan &plan);
 PlanOptions default_plan_options(int dtype, int n);
+// the default options with factored programs allowed
+PlanOptions factored_plan_options(int dtype, int n);
+PlanOptions factored_adjoint_options(int dtype, int n);
 
 // Dense fused blocks: consecutive gates on at most kDenseQubits qubits
 // multiplied (FP64, host) into one 2^k x 2^k unitary, applied as a

@@ -280,7 +280,7 @@ int qk_hsv_apply_gates(qk_hsv *h, const qk_gate *gates, size_t ng) {
     if (rc) return rc;
     // plans: each segment's gates on its local bits (local bit i = i-th lowest local qubit)
     std::vector<HostPlan> hps(segs.size());
-    const PlanOptions po = default_plan_options(h->dtype, h->L);
+    const PlanOptions po = factored_plan_options(h->dtype, h->L);
     for (size_t s = 0; s < segs.size(); ++s) {
         int rank[64];
         for (int q = 0, k = 0; q < h->n; ++q) rank[q] = (segs[s].local >> q & 1) ? k++ : -1;
@@ -291,7 +291,7 @@ int qk_hsv_apply_gates(qk_hsv *h, const qk_gate *gates, size_t ng) {
             for (int k = 0; k < x.nq; ++k) x.q[k] = rank[x.q[k]];
             g.push_back(x);
         }
-        rc = build_plan(g.data(), g.size(), h->L, po, hps[s]);
+        rc = plan_forward(g.data(), g.size(), h->L, po, hps[s]);
         if (rc) return rc;
     }
     if (h->plans.size() < segs.size()) h->plans.resize(segs.size());

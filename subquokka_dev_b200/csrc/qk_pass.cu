@@ -133,6 +133,12 @@ static int cuda_err(cudaError_t e, const char *what) {
     return fail(e == cudaErrorMemoryAllocation ? QK_ERR_OOM : QK_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
 }
 
+// factored passes (qk_fpass.cu)
+int launch_factored_pass(double2 *s, double2 *s2, int n, int r, const PassDesc &d, const TOp *ops, const double2 *coef,
+                         const int32_t *gparams, double *ggrad, cudaStream_t st);
+int launch_factored_pass(float2 *s, float2 *s2, int n, int r, const PassDesc &d, const TOp *ops, const float2 *coef,
+                         const int32_t *gparams, double *ggrad, cudaStream_t st);
+
 // Device pointers of one pass launch.
 template <typename C> struct PassArgs {
     C *s;                    // psi
@@ -203,6 +209,7 @@ static int launch_pass(C *s, int n, int r, const PassDesc &d, const TOp *ops, co
         }
         return QK_OK;
     }
+    if (d.form) return launch_factored_pass(s, s2, n, r, d, ops, coef, gparams, ggrad, st);
     // a compute pass reads its program and coefficients from device memory
     if ((d.nprog && !ops) || (d.ncoef && !coef))
         return fail(QK_ERR_ARG, "compute pass without its program in device memory");
@@ -356,7 +363,7 @@ int state_dtype(const qk_sv *sv);
 
 int apply_group_plan(qk_sv *sv, const qk_gate *gates, const int32_t *sizes, size_t ngroups) {
     HostPlan hp;
-    PlanOptions o = default_plan_options(state_dtype(sv), state_qubits(sv));
+    PlanOptions o = factored_plan_options(state_dtype(sv), state_qubits(sv));
     int rc = build_group_plan(gates, sizes, ngroups, state_qubits(sv), o, hp);
     if (rc) return rc;
     DevPlan &dp = state_scratch_plan(sv);
@@ -400,11 +407,12 @@ int qk_plan_create(const qk_gate *gates, size_t n, int nqubits, const qk_plan_op
         *out = p;
         return QK_OK;
     }
-    PlanOptions o = default_plan_options(dtype, nqubits);
-    if (opts && opts->tile_bits) o.tile_bits = opts->tile_bits;
-    if (opts && opts->reg_bits) o.reg_bits = opts->reg_bits;
+    PlanOptions o = factored_plan_options(dtype, nqubits);
+    if (opts && opts->tile_bits) o.tile_bits = o.f_tile_bits = opts->tile_bits;
+    if (opts && opts->reg_bits) o.reg_bits = o.f_reg_bits = opts->reg_bits;
+    o.f_reg_bits = std::min(o.f_reg_bits, o.f_tile_bits);
     auto *p = new qk_plan();
-    int rc = build_plan(gates, n, nqubits, o, p->hp);
+    int rc = plan_forward(gates, n, nqubits, o, p->hp);
     if (rc) {
         delete p;
         return rc;
@@ -428,9 +436,10 @@ int qk_plan_create_groups(const qk_gate *gates, const int32_t *group_sizes, size
         return qk_plan_create(gates, ng, nqubits, opts, out);
     }
     const int dtype = opts ? opts->dtype : QK_C128;
-    PlanOptions o = default_plan_options(dtype, nqubits);
-    if (opts && opts->tile_bits) o.tile_bits = opts->tile_bits;
-    if (opts && opts->reg_bits) o.reg_bits = opts->reg_bits;
+    PlanOptions o = factored_plan_options(dtype, nqubits);
+    if (opts && opts->tile_bits) o.tile_bits = o.f_tile_bits = opts->tile_bits;
+    if (opts && opts->reg_bits) o.reg_bits = o.f_reg_bits = opts->reg_bits;
+    o.f_reg_bits = std::min(o.f_reg_bits, o.f_tile_bits);
     auto *p = new qk_plan();
     int rc = build_group_plan(gates, group_sizes, ngroups, nqubits, o, p->hp);
     if (rc) {
@@ -450,7 +459,7 @@ int qk_plan_stats(const qk_plan *p, size_t *passes, size_t *program_ops, size_t 
         return QK_OK;
     }
     if (passes) *passes = p->hp.passes.size();
-    if (program_ops) *program_ops = p->hp.ops.size();
+    if (program_ops) *program_ops = p->hp.program_ops();
     if (remaps) *remaps = p->hp.nremaps;
     return QK_OK;
 }

@@ -218,18 +218,8 @@ __device__ __forceinline__ void reg_g2(C (&v)[R], const C *__restrict__ m) {
 }
 
 
-// Shared-memory layout of a tile: element j lives at swz(j), which XORs the
-// low index bits with folds of the higher ones.  A warp's lanes differ in
-// three (complex128) or four (complex64) consecutive thread bits wherever the
-// register qubits sit, and the fold sends those bits to distinct banks, so
-// the re-mappings stay (nearly) conflict-free.
-template <typename C> __device__ __forceinline__ uint32_t swz(uint32_t j) {
-    if constexpr (sizeof(C) == 16) {
-        return j ^ (((j >> 3) ^ (j >> 6) ^ (j >> 9) ^ (j >> 12)) & 7u);
-    } else {
-        return j ^ (((j >> 4) ^ (j >> 8) ^ (j >> 12)) & 15u);
-    }
-}
+// Shared-memory layout of a tile (tile_swizzle in qk_internal.h).
+template <typename C> __device__ __forceinline__ uint32_t swz(uint32_t j) { return tile_swizzle(j, sizeof(C) == 16); }
 
 // Asynchronous global -> shared copy of one amplitude (cp.async, sm_80+).
 template <typename C> __device__ __forceinline__ void cp_async_amp(C *dst_smem, const C *src) {

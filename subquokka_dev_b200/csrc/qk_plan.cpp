@@ -64,9 +64,14 @@ namespace {
 
 int low_bits(int dtype) { return dtype == QK_C128 ? 3 : 4; }  // 128-byte runs
 
+}  // namespace
+
 // Most tile bits of a permutation pass (qk_pass.cu stages such a tile in
 // shared memory in one buffer).
 int perm_tile_bits(int dtype) { return dtype == QK_C128 ? 13 : 14; }
+
+namespace {
+
 constexpr int kPermMinTileBits = 10;
 
 void push_c(HostPlan &p, double re, double im) {
@@ -558,6 +563,8 @@ int lower_all(const qk_gate *gates, size_t ng, int n, std::vector<Op> &ops) {
     return QK_OK;
 }
 
+}  // namespace
+
 // Leading state bits always in the tile; two tile bits stay free for the
 // qubits of any single gate, so every pass takes at least one gate.
 int pass_low_bits(const PlanOptions &o, int n) {
@@ -582,8 +589,6 @@ int check_options(const PlanOptions &o, int n) {
     if (bytes > (200u << 10)) return fail(QK_ERR_ARG, "tile of %zu bytes exceeds shared memory", bytes);
     return QK_OK;
 }
-
-}  // namespace
 
 int build_plan(const qk_gate *gates, size_t ng, int n, const PlanOptions &o, HostPlan &plan) {
     int rc = check_options(o, n);
@@ -929,19 +934,6 @@ int build_dense_blocks(const qk_gate *gates, size_t ng, int n, int width, int dt
         }
     dense_partition(*best_list, n, width, best_seeds, true, blocks);
     return QK_OK;
-}
-
-int build_group_plan(const qk_gate *gates, const int32_t *sizes, size_t ngroups, int n, const PlanOptions &o,
-                     HostPlan &plan) {
-    size_t ng = 0;
-    for (size_t g = 0; g < ngroups; ++g) {
-        if (sizes[g] < 0) return fail(QK_ERR_ARG, "group %zu has negative size", g);
-        ng += (size_t)sizes[g];
-    }
-    // The groups bound nothing here: a tile can hold any qubits, and VSWAP
-    // groups become renamings, so the gates of all groups are planned as one
-    // gate list.
-    return build_plan(gates, ng, n, o, plan);
 }
 
 }  // namespace qk
