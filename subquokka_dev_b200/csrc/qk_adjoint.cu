@@ -26,6 +26,7 @@
 #include "qk_device.h"
 #include "qk_internal.h"
 #include "qk_kernels.cuh"
+#include "qk_pass_device.cuh"
 
 namespace qk {
 
@@ -101,6 +102,172 @@ __global__ void __launch_bounds__(kRedThreads) k_pauli_apply(C *__restrict__ out
             im += o.y;
         }
         out[j] = mk<C>(re, im);
+    }
+}
+
+// Pauli groups by tiles: all groups whose X masks lie in the tile's bits, from
+// one read of the state.  One group a sweep is bound by HBM -- H = sum J Z Z +
+// sum h X on 27 qubits took 28 sweeps of a 2 GiB state, 18.2 ms -- and the
+// groups of a tile of 2^T amplitudes with the lowest L bits share theirs
+// (T - L qubits' X terms a sweep: four sweeps there).
+constexpr int kTileGroups = 24, kTileTerms = 64;
+constexpr int kTileSlots = 2;   // elements a thread: 2^kTileSlots
+struct PauliTile {
+    PassDesc d;                            // T, L, bpos
+    int ngroups;
+    int16_t term0[kTileGroups + 1];        // terms of group g: term0[g] .. term0[g + 1]
+    int nsimple;                           // groups of one term without Z: its coefficient (real), and
+    double scoef[kTileGroups];             // the places of its partners, an XOR of byte offsets
+    uint32_t splace[kTileGroups];
+    uint32_t xplace[kTileGroups];          // the same of the other groups' partners
+    uint64_t x[kTileGroups];               // and their X masks over the state's bits
+    double coef[kTileTerms];
+    uint64_t z[kTileTerms];
+    uint8_t ipow[kTileTerms];
+};
+
+// out (+)= sum of the groups' P psi (out may be null), acc += Re <psi| them >
+//
+// The sign of term k at an amplitude is the parity of its index & z[k], a sum
+// of the parities of the tile's, the thread's and the element's parts: three
+// 64-bit words with a bit a term, of which only the tile's is made anew for a
+// tile (a lane a term).  With the parities taken term by term, POPC bound the
+// kernel (27 qubits, 53 terms: 7.6 ms).  Groups of one X string, the common
+// case, run ahead of the others in a loop of their own.
+template <typename C>
+__global__ void __launch_bounds__(kRedThreads, 2) k_pauli_tile(C *__restrict__ out, const C *__restrict__ psi, uint64_t ntiles,
+                                                            const __grid_constant__ PauliTile t, int accumulate,
+                                                            double *acc) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];   // the tile
+    const uint32_t NT = blockDim.x, N = 1u << t.d.T, tid = threadIdx.x, lane = tid & 31;
+    constexpr int E = 1 << kTileSlots;
+    const int nterms = t.term0[t.ngroups];
+    // element u of the thread: tid + u NT; its offset is linear in u's bits
+    const uint64_t off_t = tid < N ? pass_off(tid, t.d) : 0;
+    uint64_t off_u[kTileSlots];
+    uint64_t sg_t = 0, sg_u[kTileSlots];   // bit k: parity of the part & z[k]
+#pragma unroll
+    for (int b = 0; b < kTileSlots; ++b) {
+        off_u[b] = (NT << b) < N ? pass_off(NT << b, t.d) : 0;
+        sg_u[b] = 0;
+    }
+    for (int k = 0; k < nterms; ++k) {
+        const uint64_t z = t.z[k];
+        sg_t |= (uint64_t)(__popcll(off_t & z) & 1) << k;
+#pragma unroll
+        for (int b = 0; b < kTileSlots; ++b) sg_u[b] |= (uint64_t)(__popcll(off_u[b] & z) & 1) << k;
+    }
+    // of the lane's terms lane and lane + 32: z, and whether its constant part
+    // (x & z, the sign of i^ipow) is negative
+    uint64_t z0 = 0, z1 = 0;
+    int c0 = 0, c1 = 0;
+    for (int g = 0; g < t.ngroups; ++g)
+        for (int k = t.term0[g]; k < t.term0[g + 1]; ++k) {
+            const int c = (__popcll(t.x[g] & t.z[k]) & 1) ^ (t.ipow[k] >> 1);
+            if (k == (int)lane) z0 = t.z[k], c0 = c;
+            if (k == (int)lane + 32) z1 = t.z[k], c1 = c;
+        }
+    uint32_t place[E];   // (elements past a small tile's end: those of its start)
+#pragma unroll
+    for (int u = 0; u < E; ++u) place[u] = swz<C>((tid + u * NT) & (N - 1)) * (uint32_t)sizeof(C);
+    double sum = 0;
+    uint64_t off[E];
+#pragma unroll
+    for (int u = 0; u < E; ++u) {
+        off[u] = off_t;
+#pragma unroll
+        for (int b = 0; b < kTileSlots; ++b)
+            if ((u >> b) & 1) off[u] |= off_u[b];
+    }
+    // a tile's amplitudes are loaded while the one before it is worked on
+    C next[E];
+    uint64_t base = 0;
+    auto load = [&](uint64_t o) {
+        base = pass_base(o, t.d);
+#pragma unroll
+        for (int u = 0; u < E; ++u)
+            if (tid + u * NT < N) next[u] = psi[base | off[u]];
+    };
+    if (blockIdx.x < ntiles) load(blockIdx.x);
+    for (uint64_t o = blockIdx.x; o < ntiles; o += gridDim.x) {
+        const uint64_t here = base;
+        C v[E];
+#pragma unroll
+        for (int u = 0; u < E; ++u) {
+            v[u] = next[u];
+            if (tid + u * NT < N) *reinterpret_cast<C *>(smem_raw + place[u]) = v[u];
+        }
+        __syncthreads();
+        if (o + gridDim.x < ntiles) load(o + gridDim.x);
+        uint64_t sg[E];
+        const uint64_t sg_tile =
+            (uint64_t)__ballot_sync(0xffffffffu, (__popcll(here & z1) ^ c1) & 1) << 32 |
+            __ballot_sync(0xffffffffu, (__popcll(here & z0) ^ c0) & 1);
+#pragma unroll
+        for (int u = 0; u < E; ++u) {
+            sg[u] = sg_tile ^ sg_t;
+#pragma unroll
+            for (int b = 0; b < kTileSlots; ++b)
+                if ((u >> b) & 1) sg[u] ^= sg_u[b];
+        }
+        double re[E], im[E];
+#pragma unroll
+        for (int u = 0; u < E; ++u) re[u] = im[u] = 0;
+        // += (fr + i fi) b, the group's factor at the element
+        auto add = [&](int u, const C b, double fr, double fi) {
+            re[u] += fr * (double)b.x - fi * (double)b.y;
+            im[u] += fr * (double)b.y + fi * (double)b.x;
+        };
+#pragma unroll 4
+        for (int g = 0; g < t.nsimple; ++g) {
+            const double c = t.scoef[g];
+            const uint32_t xp = t.splace[g];
+#pragma unroll
+            for (int u = 0; u < E; ++u) {
+                const C b = *reinterpret_cast<const C *>(smem_raw + (place[u] ^ xp));
+                re[u] += c * (double)b.x;
+                im[u] += c * (double)b.y;
+            }
+        }
+        for (int g = 0; g < t.ngroups; ++g) {
+            const int t0 = t.term0[g], t1 = t.term0[g + 1];
+            const uint32_t xp = t.xplace[g];
+            double fr[E], fi[E];
+#pragma unroll
+            for (int u = 0; u < E; ++u) fr[u] = fi[u] = 0;
+            for (int k = t0; k < t1; ++k) {
+                const double c = t.coef[k];
+                const bool odd = t.ipow[k] & 1;
+#pragma unroll
+                for (int u = 0; u < E; ++u) {
+                    const uint32_t w = k < 32 ? (uint32_t)sg[u] : (uint32_t)(sg[u] >> 32);
+                    const double s = __hiloint2double(__double2hiint(c) ^ (int)((w >> (k & 31)) << 31), __double2loint(c));
+                    if (odd) fi[u] += s;
+                    else fr[u] += s;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < E; ++u)
+                add(u, *reinterpret_cast<const C *>(smem_raw + (place[u] ^ xp)), fr[u], fi[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < E; ++u)
+            if (tid + u * NT < N) {
+                sum += (double)v[u].x * re[u] + (double)v[u].y * im[u];
+                if (out) {
+                    C *p = out + (here | off[u]);
+                    if (accumulate) {
+                        re[u] += p->x;
+                        im[u] += p->y;
+                    }
+                    *p = mk<C>(re[u], im[u]);
+                }
+            }
+        __syncthreads();
+    }
+    if (acc) {
+        sum = block_sum(sum);
+        if (threadIdx.x == 0) atomicAdd(acc, sum);
     }
 }
 
@@ -198,30 +365,117 @@ static int group_terms(const qk_pauli_term *terms, size_t nterms, int n, std::ve
     return QK_OK;
 }
 
-template <typename C>
-static int expval_t(const C *psi, int n, const std::vector<PauliGroup> &groups, double *dacc, cudaStream_t st) {
-    const uint64_t namp = 1ull << n;
-    for (const auto &g : groups) {
-        k_pauli_expval<C><<<red_grid(namp), kRedThreads, 0, st>>>(psi, namp, g, dacc);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return cuda_err(e, "k_pauli_expval");
+// Tile bits of k_pauli_tile: kRedThreads threads with 2^kTileSlots elements
+// each, 16 KB of complex128.
+constexpr int kPauliTileBits = 8 + kTileSlots;
+static_assert(1 << (kPauliTileBits - kTileSlots) == kRedThreads, "elements a thread");
+
+// The groups whose X masks fit a tile, cut into tiles; the others stay in
+// `flat` (one sweep each).
+//
+// A complex64 H psi is written group by group, each sum rounded to 24 bits,
+// as the gradients of complex64 sweeps have been computed: with one rounding
+// a tile they changed by 6e-8.
+static void tile_groups(const std::vector<PauliGroup> &groups, int n, int dtype, bool apply, std::vector<PauliTile> &tiles,
+                        std::vector<PauliGroup> &flat) {
+    if (apply && dtype == QK_C64) {
+        flat = groups;
+        return;
     }
-    return QK_OK;
+    const int T = std::min(n, kPauliTileBits), L = std::min(T, dtype == QK_C128 ? 3 : 4);   // 128-byte runs
+    const uint64_t low = (1ull << L) - 1;
+    std::vector<const PauliGroup *> left;
+    for (const PauliGroup &g : groups) {
+        if (__builtin_popcountll(g.x | low) > T) flat.push_back(g);
+        else left.push_back(&g);
+    }
+    std::stable_sort(left.begin(), left.end(), [](const PauliGroup *a, const PauliGroup *b) { return a->x < b->x; });
+    while (!left.empty()) {
+        PauliTile t;
+        std::memset(&t, 0, sizeof t);
+        uint64_t bits = low;
+        std::vector<const PauliGroup *> take, rest;
+        int nt = 0;
+        for (const PauliGroup *g : left) {
+            const bool ok = (int)take.size() < kTileGroups && nt + g->nterms <= kTileTerms &&
+                            __builtin_popcountll(bits | g->x) <= T;
+            (ok ? take : rest).push_back(g);
+            if (ok) bits |= g->x, nt += g->nterms;
+        }
+        for (int q = 0; __builtin_popcountll(bits) < T; ++q) bits |= 1ull << q;
+        t.d.T = T;
+        for (int q = 0, k = 0; q < n; ++q)
+            if ((bits >> q) & 1) t.d.bpos[k++] = q;
+        while (t.d.L < T && t.d.bpos[t.d.L] == t.d.L) ++t.d.L;
+        int k = 0;
+        for (const PauliGroup *g : take) {
+            uint32_t xl = 0;
+            for (int b = 0; b < T; ++b) xl |= (uint32_t)((g->x >> t.d.bpos[b]) & 1) << b;
+            const uint32_t place = tile_swizzle(xl, dtype == QK_C128) * (dtype == QK_C128 ? 16 : 8);
+            if (g->nterms == 1 && !g->z[0]) {
+                t.scoef[t.nsimple] = g->coef[0];
+                t.splace[t.nsimple++] = place;
+                continue;
+            }
+            t.x[t.ngroups] = g->x;
+            t.xplace[t.ngroups] = place;
+            t.term0[t.ngroups++] = (int16_t)k;
+            for (int i = 0; i < g->nterms; ++i, ++k) {
+                t.coef[k] = g->coef[i];
+                t.z[k] = g->z[i];
+                t.ipow[k] = (uint8_t)g->ipow[i];
+            }
+        }
+        t.term0[t.ngroups] = (int16_t)k;
+        tiles.push_back(t);
+        left.swap(rest);
+    }
 }
 
+// out = H psi (out may be null) and, with acc (zero before), *acc = <H>.
+static size_t pauli_sweeps(const std::vector<PauliGroup> &groups, int n, int dtype) {
+    std::vector<PauliTile> tiles;
+    std::vector<PauliGroup> flat;
+    tile_groups(groups, n, dtype, true, tiles, flat);
+    return tiles.size() + flat.size();
+}
+
+// out = H psi (out may be null) and, with acc (zero before), *acc = <H>.
 template <typename C>
-static int apply_h_t(C *out, const C *psi, int n, const std::vector<PauliGroup> &groups, cudaStream_t st) {
+static int pauli_sum_t(C *out, const C *psi, int n, const std::vector<PauliGroup> &groups, double *acc, cudaStream_t st) {
     const uint64_t namp = 1ull << n;
     if (groups.empty()) {
-        cudaError_t e = cudaMemsetAsync(out, 0, sizeof(C) * namp, st);
+        cudaError_t e = out ? cudaMemsetAsync(out, 0, sizeof(C) * namp, st) : cudaSuccess;
         return e == cudaSuccess ? QK_OK : cuda_err(e, "memset");
     }
-    for (size_t i = 0; i < groups.size(); ++i) {
-        k_pauli_apply<C><<<red_grid(namp), kRedThreads, 0, st>>>(out, psi, namp, groups[i], i > 0);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return cuda_err(e, "k_pauli_apply");
+    std::vector<PauliTile> tiles;
+    std::vector<PauliGroup> flat;
+    tile_groups(groups, n, sizeof(C) == sizeof(double2) ? QK_C128 : QK_C64, out != nullptr, tiles, flat);
+    int done = 0;
+    for (const PauliTile &t : tiles) {
+        const unsigned threads = std::min(kRedThreads, std::max(32, (1 << t.d.T) >> kTileSlots));
+        const size_t smem = sizeof(C) << t.d.T;
+        int mb = 0;
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&mb, k_pauli_tile<C>, (int)threads, smem);
+        if (e != cudaSuccess || mb < 1) mb = 1;
+        const uint64_t ntiles = namp >> t.d.T;
+        const unsigned grid = (unsigned)std::min<uint64_t>(ntiles, (uint64_t)device_sms() * mb);
+        k_pauli_tile<C><<<grid, threads, smem, st>>>(out, psi, ntiles, t, done++ > 0, acc);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return cuda_err(e, "k_pauli_tile");
     }
-    return QK_OK;
+    for (const PauliGroup &g : flat) {
+        if (out) k_pauli_apply<C><<<red_grid(namp), kRedThreads, 0, st>>>(out, psi, namp, g, done++ > 0);
+        else k_pauli_expval<C><<<red_grid(namp), kRedThreads, 0, st>>>(psi, namp, g, acc);
+    }
+    if (out && acc && !flat.empty()) {
+        // <H> from all of H psi
+        cudaError_t e = cudaMemsetAsync(acc, 0, sizeof(double), st);
+        if (e != cudaSuccess) return cuda_err(e, "clear accumulator");
+        k_dot_re<C><<<red_grid(namp), kRedThreads, 0, st>>>(psi, out, namp, acc);
+    }
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? QK_OK : cuda_err(e, "k_pauli");
 }
 
 // generator of a trainable gate: 1 X (RX), 2 Y (RY), 3 Z (RZ), 0 not trainable
@@ -267,7 +521,7 @@ static int adjoint_t(C *psi, int n, int dtype, const qk_gate *gates, size_t ng, 
     if (e == cudaSuccess) e = cudaEventRecord(ws.ev0, st);
     if (e != cudaSuccess) return cuda_err(e, "sweep timing events");
     ws.last_fwd = ws.last_bwd = (int)ng;   // one launch per gate each way
-    ws.last_other = (int)(groups.size() + 1 + 3 * cpos.size());
+    ws.last_other = (int)(pauli_sweeps(groups, n, dtype) + 3 * cpos.size());
     ws.last_bytes = 0;                     // not counted for the per-gate sweep
     e = cudaMemsetAsync(dacc, 0, nacc * sizeof(double), st);
     if (e != cudaSuccess) return cuda_err(e, "clear accumulators");
@@ -284,9 +538,8 @@ static int adjoint_t(C *psi, int n, int dtype, const qk_gate *gates, size_t ng, 
         if (rc) return rc;
     }
     // lambda = H psi, <H> = Re<psi|lambda>
-    rc = apply_h_t<C>(lam, psi, n, groups, st);
+    rc = pauli_sum_t<C>(lam, psi, n, groups, dacc + nparams, st);
     if (rc) return rc;
-    k_dot_re<C><<<red_grid(namp), kRedThreads, 0, st>>>(psi, lam, namp, dacc + nparams);
     // backward
     for (size_t i = ng; i-- > 0;) {
         Op inv = ops[i];
@@ -402,10 +655,10 @@ static int adjoint_fused_t(C *psi, int n, int dtype, const qk_gate *gates, size_
         ws.last_bwd += (int)bwd[sgi].passes.size();
     }
     const double S = (double)bytes;
-    const double ng_h = groups.empty() ? 1.0 : (double)groups.size();
-    ws.last_other = (int)(ng_h + 1 + 3 * (nseg - 1));
-    ws.last_bytes = 2 * S * ws.last_fwd + 4 * S * ws.last_bwd + (groups.empty() ? S : 2 * S + 3 * S * (ng_h - 1)) +
-                    2 * S + 3 * 2 * S * (double)(nseg - 1);
+    const double nh = (double)std::max<size_t>(1, pauli_sweeps(groups, n, dtype));
+    ws.last_other = (int)(nh + 3 * (nseg - 1));
+    ws.last_bytes = 2 * S * ws.last_fwd + 4 * S * ws.last_bwd + (groups.empty() ? S : 2 * S + 3 * S * (nh - 1)) +
+                    3 * 2 * S * (double)(nseg - 1);
     // forward
     for (size_t sgi = 0; sgi < nseg; ++sgi) {
         if (sgi > 0) {
@@ -415,9 +668,8 @@ static int adjoint_fused_t(C *psi, int n, int dtype, const qk_gate *gates, size_
         int rc = run_forward_plan(psi, fwd[sgi], ws.plans[2 * sgi], st);
         if (rc) return rc;
     }
-    int rc = apply_h_t<C>(lam, psi, n, groups, st);
+    int rc = pauli_sum_t<C>(lam, psi, n, groups, dacc + nparams, st);
     if (rc) return rc;
-    k_dot_re<C><<<red_grid(namp), kRedThreads, 0, st>>>(psi, lam, namp, dacc + nparams);
     // backward
     for (size_t sgi = nseg; sgi-- > 0;) {
         rc = run_adjoint_plan(psi, lam, dtype, bwd[sgi], ws.plans[2 * sgi + 1], dacc, st);
@@ -472,8 +724,9 @@ int qk_expval_pauli(qk_sv *sv, const qk_pauli_term *terms, size_t nterms, double
     double *dacc = ws.acc;
     e = cudaMemsetAsync(dacc, 0, sizeof(double), st);
     if (e != cudaSuccess) return cuda_err(e, "clear accumulator");
-    rc = state_dtype(sv) == QK_C128 ? expval_t<double2>((const double2 *)state_ptr(sv), n, groups, dacc, st)
-                                    : expval_t<float2>((const float2 *)state_ptr(sv), n, groups, dacc, st);
+    rc = state_dtype(sv) == QK_C128
+             ? pauli_sum_t<double2>(nullptr, (const double2 *)state_ptr(sv), n, groups, dacc, st)
+             : pauli_sum_t<float2>(nullptr, (const float2 *)state_ptr(sv), n, groups, dacc, st);
     if (!rc) {
         e = cudaMemcpyAsync(out, dacc, sizeof(double), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
