@@ -620,12 +620,24 @@ static int adjoint_fused_t(C *psi, int n, int dtype, const qk_gate *gates, size_
     // 17.9, its two-state passes being most of it
     const PlanOptions fo = dtype == QK_C128 ? factored_plan_options(dtype, n) : default_plan_options(dtype, n);
     const PlanOptions bo = factored_adjoint_options(dtype, n);
-    for (size_t sgi = 0; sgi < nseg; ++sgi) {
+    // planning takes longer than the sweep of a small state: every segment's
+    // two plans on threads of their own (13 qubits, 190 gates: 1.2 -> 0.4 ms;
+    // 26 qubits, 924 gates: 12 -> 3 ms)
+    auto plan_one = [&](size_t k) {
+        const size_t sgi = k / 2, cnt = cut[sgi + 1] - cut[sgi];
         const qk_gate *g = gates + cut[sgi];
-        const size_t cnt = cut[sgi + 1] - cut[sgi];
-        int rc = plan_forward(g, cnt, n, fo, fwd[sgi]);
-        if (!rc) rc = plan_adjoint(g, cnt, pidx ? pidx + cut[sgi] : nullptr, n, bo, bwd[sgi]);
+        return k % 2 ? plan_adjoint(g, cnt, pidx ? pidx + cut[sgi] : nullptr, n, bo, bwd[sgi])
+                     : plan_forward(g, cnt, n, fo, fwd[sgi]);
+    };
+    if (ng >= 100) {
+        int rc = run_tasks(2 * nseg, plan_one);
         if (rc) return rc;
+    }
+    for (size_t sgi = 0; sgi < nseg; ++sgi) {
+        for (size_t k = 2 * sgi; k < 2 * sgi + 2 && ng < 100; ++k) {
+            int rc = plan_one(k);
+            if (rc) return rc;
+        }
         for (int32_t p : bwd[sgi].grad_params)
             if (p < 0 || (size_t)p >= nparams) return fail(QK_ERR_ARG, "parameter %d >= %zu", p, nparams);
     }

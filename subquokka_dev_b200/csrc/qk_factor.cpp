@@ -17,14 +17,46 @@
 //   indices) a thread's amplitudes carry, and the next re-mapping writes them
 //   to their new places.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <complex>
 #include <cstring>
+#include <new>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "qk_internal.h"
 
 namespace qk {
+
+int run_tasks(size_t n, const std::function<int(size_t)> &task) {
+    std::vector<int> rc(n, QK_OK);
+    std::vector<std::string> what(n);
+    std::atomic<size_t> next{0};
+    auto work = [&]() {
+        for (size_t i = next++; i < n; i = next++) {
+            try {
+                rc[i] = task(i);
+            } catch (const std::bad_alloc &) {
+                rc[i] = fail(QK_ERR_OOM, "out of host memory");
+            }
+            if (rc[i]) what[i] = qk_last_error();
+        }
+    };
+    std::vector<std::thread> pool;
+    const size_t cores = std::max(1u, std::thread::hardware_concurrency());
+    try {
+        for (size_t t = 1; t < std::min(n, cores); ++t) pool.emplace_back(work);
+    } catch (const std::system_error &) {
+        // no more threads: those that run, and this one, take the tasks
+    }
+    work();
+    for (std::thread &t : pool) t.join();
+    for (size_t i = 0; i < n; ++i)
+        if (rc[i]) return fail(rc[i], "%s", what[i].c_str());
+    return QK_OK;
+}
 
 // Tile and register bits of factored passes.  complex128: 1024-amplitude
 // tiles, 16 amplitudes a thread (64 threads, eight CTAs an SM); with 2048 the
@@ -1003,21 +1035,33 @@ int build_best(const std::vector<std::vector<Op>> &lists, const std::vector<cl> 
     empty.T = o.f_tile_bits;
     empty.r = o.f_reg_bits;
     empty.nstates = nstates;
+    std::vector<Candidate> all(4 * lists.size());
+    auto candidate = [&](size_t k) {
+        const size_t list = k / 4, variant = k % 4;
+        Candidate &c = all[k];
+        c.list = list;
+        c.ops = lists[list];
+        if (variant % 2) asap_order(c.ops, n);
+        HostPlan hp = empty;
+        Builder b{c.ops, n, o.f_tile_bits, o.f_reg_bits, L, hp, o, variant >= 2, scale[list], scaled[list] != 0};
+        b.partition();
+        c.parts.swap(b.parts);
+        return (int)QK_OK;
+    };
+    // (a thread costs some 30 us to start, a candidate of a few hundred ops more)
+    const bool threads = o.threads && lists[0].size() >= 100;
+    for (size_t k = 0; k < all.size() && !threads; ++k) candidate(k);
+    if (threads) {
+        int rc = run_tasks(all.size(), candidate);
+        if (rc) return rc;
+    }
     bool have = false, two = false;
-    for (size_t list = 0; list < lists.size(); ++list)
-        for (int variant = 0; variant < 4; ++variant) {
-            Candidate c;
-            c.list = list;
-            c.ops = lists[list];
-            if (variant % 2) asap_order(c.ops, n);
-            Builder b{c.ops, n, o.f_tile_bits, o.f_reg_bits, L, empty, o, variant >= 2, scale[list], scaled[list] != 0};
-            b.partition();
-            if (have && b.parts.size() > first.parts.size()) continue;
-            c.parts.swap(b.parts);
-            two = have && c.parts.size() == first.parts.size();
-            std::swap(two ? last : first, c);
-            have = true;
-        }
+    for (Candidate &c : all) {
+        if (have && c.parts.size() > first.parts.size()) continue;
+        two = have && c.parts.size() == first.parts.size();
+        std::swap(two ? last : first, c);
+        have = true;
+    }
     for (Candidate *c : {&first, &last}) {
         if (c == &last && !two) break;
         HostPlan hp = empty;

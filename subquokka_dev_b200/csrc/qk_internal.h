@@ -3,6 +3,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -42,6 +43,11 @@ struct Op {
 // Thread-local error message; returns code so callers can `return fail(...)`.
 int fail(int code, const char *fmt, ...) __attribute__((format(printf, 2, 3)));
 void clear_error();
+
+// task(0) .. task(n - 1) on up to n host threads, this one among them (all of
+// them on this one where no thread can be had).  Returns the first failing
+// task's code, with its message.
+int run_tasks(size_t n, const std::function<int(size_t)> &task);
 
 // Lower a parsed gate to a kernel op (host, FP64).
 int lower_gate(const qk_gate &g, Op &op);
@@ -194,6 +200,7 @@ struct PlanOptions {
     // plan_forward / plan_adjoint: tile and register bits of factored programs,
     // which are made where they can be (0: general programs only)
     int f_tile_bits = 0, f_reg_bits = 0;
+    int threads = 0;      // 1: the factored planner tries its candidates on several host threads
 };
 
 // The fused plan of a flat gate list / of a backward sweep as the engine runs

@@ -364,6 +364,7 @@ int state_dtype(const qk_sv *sv);
 int apply_group_plan(qk_sv *sv, const qk_gate *gates, const int32_t *sizes, size_t ngroups) {
     HostPlan hp;
     PlanOptions o = factored_plan_options(state_dtype(sv), state_qubits(sv));
+    o.threads = 1;   // planned on every call
     int rc = build_group_plan(gates, sizes, ngroups, state_qubits(sv), o, hp);
     if (rc) return rc;
     DevPlan &dp = state_scratch_plan(sv);
@@ -411,6 +412,7 @@ int qk_plan_create(const qk_gate *gates, size_t n, int nqubits, const qk_plan_op
     if (opts && opts->tile_bits) o.tile_bits = o.f_tile_bits = opts->tile_bits;
     if (opts && opts->reg_bits) o.reg_bits = o.f_reg_bits = opts->reg_bits;
     o.f_reg_bits = std::min(o.f_reg_bits, o.f_tile_bits);
+    o.threads = 1;
     auto *p = new qk_plan();
     int rc = plan_forward(gates, n, nqubits, o, p->hp);
     if (rc) {
@@ -440,6 +442,7 @@ int qk_plan_create_groups(const qk_gate *gates, const int32_t *group_sizes, size
     if (opts && opts->tile_bits) o.tile_bits = o.f_tile_bits = opts->tile_bits;
     if (opts && opts->reg_bits) o.reg_bits = o.f_reg_bits = opts->reg_bits;
     o.f_reg_bits = std::min(o.f_reg_bits, o.f_tile_bits);
+    o.threads = 1;
     auto *p = new qk_plan();
     int rc = build_group_plan(gates, group_sizes, ngroups, nqubits, o, p->hp);
     if (rc) {

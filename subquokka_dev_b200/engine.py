@@ -16,7 +16,7 @@ from typing import Iterable, Sequence
 import numpy as np
 
 from . import _lib
-from ._lib import GATE_KINDS, KIND_NAMES, QK_C64, QK_C128, QkConfig, QkGate, check
+from ._lib import GATE_KINDS, KIND_NAMES, QK_C64, QK_C128, QK_MAX_TARGETS, QkConfig, QkGate, check
 
 DTYPES = {"c128": QK_C128, "c64": QK_C64, QK_C128: QK_C128, QK_C64: QK_C64}
 
@@ -70,6 +70,15 @@ class Circuit:
         self.ngroups = len(gs)
 
     @classmethod
+    def blank(cls, ngates: int) -> "Circuit":
+        """A flat circuit of ngates zeroed records, to be filled (gate_records)."""
+        c = cls([])
+        c.gates = (QkGate * max(1, ngates))()
+        c.ngates = c.ngroups = ngates
+        c.group_sizes = (c_int32 * max(1, ngates))(*([1] * ngates))
+        return c
+
+    @classmethod
     def _from_handle(cls, h: c_void_p) -> "Circuit":
         lib = _lib.load()
         try:
@@ -110,6 +119,16 @@ class Circuit:
                 lines += [gate_line(self.gates[k + j]) for j in range(n)]
                 k += n
         return "\n".join(lines) + "\n" if lines else ""
+
+
+GATE_RECORD = np.dtype([("kind", np.int32), ("nq", np.int32), ("q", np.int32, QK_MAX_TARGETS), ("param", np.float64),
+                        ("coeff", np.float64, 32)], align=True)
+assert GATE_RECORD.itemsize == ctypes.sizeof(QkGate)
+
+
+def gate_records(circuit: Circuit) -> np.ndarray:
+    """The circuit's gate records as a structured array over the same memory."""
+    return np.frombuffer(circuit.gates, dtype=GATE_RECORD, count=circuit.ngates)
 
 
 def chunk_groups(circuit: Circuit, n: int, chunk_qbit: int = 12) -> Circuit:
