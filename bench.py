@@ -723,7 +723,7 @@ def our_arm(args, rank, world):
                 "kernel_share": {k: v / tot for k, v in sorted(shares.items())},
                 "kernel_gbs": {k: (2 * S if k.startswith("k_dense1") else S // 2) / (statistics.mean(v) / 1e3) / 1e9
                                for k, v in per_kernel.items()}}
-    launches = args.steps * (circ.ngates + 1)
+    launches = args.steps * (gate_launches(circ) + 1)
     # the fused forms and the other workloads are single-GPU measurements:
     # a run on N > 1 GPUs (replicas of the timed step) skips them and runs
     # the two multi-GPU legs instead, so that it holds the GPUs briefly

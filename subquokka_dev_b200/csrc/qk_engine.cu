@@ -140,17 +140,64 @@ int launch_gate_op(void *state, int n, int dtype, const Op &op, cudaStream_t st)
     return dtype == QK_C128 ? launch_op<double2>((double2 *)state, n, op, st) : launch_op<float2>((float2 *)state, n, op, st);
 }
 
+// ops[0..n) in order, runs of diagonal ops as one sweep each.
+template <typename C>
+static int launch_ops(C *s, int n, const Op *ops, size_t count, cudaStream_t st) {
+    for (size_t i = 0; i < count;) {
+        size_t k = i;
+        while (k < count && k - i < (size_t)kRunGates && op_is_diagonal(ops[k])) ++k;
+        if (k - i < 2) {
+            int rc = launch_op<C>(s, n, ops[i++], st);
+            if (rc) return rc;
+            continue;
+        }
+        DiagRun<C> r;
+        r.n = (int)(k - i);
+        uint64_t common = ~0ull;
+        for (int g = 0; g < r.n; ++g) {
+            const Op &op = ops[i + g];
+            const bool phase = op.kind == OP_PHASE1 || op.kind == OP_PHASE2;
+            r.mask[g] = 0;
+            r.qa[g] = (int16_t)op.q[0];
+            r.qb[g] = (int16_t)(op.nq > 1 ? op.q[1] : op.q[0]);
+            if (phase) {
+                r.mask[g] = 1ull << r.qa[g] | 1ull << r.qb[g];
+                r.d[g][3] = mk<C>(op.m[0], op.m[1]);
+            } else {
+                // one qubit: entries 0 and 3 (qa = qb)
+                for (int d = 0; d < (op.nq > 1 ? 4 : 2); ++d)
+                    r.d[g][op.nq > 1 ? d : 3 * d] = mk<C>(op.m[2 * d], op.m[2 * d + 1]);
+            }
+            common &= r.mask[g];
+        }
+        const int t = common ? __builtin_ctzll(common) : -1;
+        const uint64_t items = (1ull << n) >> (t >= 0);
+        if (n <= 32) k_diag_run<C, uint32_t><<<sweep_blocks(items), kBlock, 0, st>>>(s, items, t, r);
+        else k_diag_run<C, uint64_t><<<sweep_blocks(items), kBlock, 0, st>>>(s, items, t, r);
+        QK_CUDA(cudaGetLastError());
+        i = k;
+    }
+    return QK_OK;
+}
+
 template <typename C>
 static int apply_gates_t(C *s, int n, const qk_gate *gates, size_t ng, cudaStream_t st) {
-    for (size_t i = 0; i < ng; ++i) {
-        Op op;
-        int rc = lower_gate(gates[i], op);
-        if (rc) return rc;
-        for (int k = 0; k < op.nq; ++k)
-            if (op.q[k] < 0 || op.q[k] >= n)
-                return fail(QK_ERR_QUBIT, "gate %zu: qubit %d outside a %d-qubit state", i, op.q[k], n);
-        rc = launch_op<C>(s, n, op, st);
-        if (rc) return rc;
+    // gates are lowered a window at a time; those before a gate in error are
+    // applied, as if one by one
+    Op ops[2 * kRunGates];
+    for (size_t i = 0; i < ng;) {
+        size_t k = 0;
+        int rc = QK_OK;
+        for (; k < 2 * kRunGates && i < ng && !rc; ++i) {
+            Op &op = ops[k];
+            rc = lower_gate(gates[i], op);
+            for (int j = 0; j < op.nq && !rc; ++j)
+                if (op.q[j] < 0 || op.q[j] >= n)
+                    rc = fail(QK_ERR_QUBIT, "gate %zu: qubit %d outside a %d-qubit state", i, op.q[j], n);
+            k += !rc;
+        }
+        const int lrc = launch_ops<C>(s, n, ops, k, st);
+        if (rc || lrc) return lrc ? lrc : rc;
     }
     return QK_OK;
 }
@@ -393,7 +440,12 @@ int qk_graph_create(qk_sv *sv, const qk_gate *gates, size_t n, qk_graph **out) {
         return cuda_fail(e, "cudaStreamBeginCapture");
     }
     int rc = QK_OK;
-    for (size_t i = 0; i < n && !rc; ++i) rc = launch_gate_op(sv->d, sv->n, sv->dtype, ops[i], cs);
+    // the windows of apply_gates_t, so that a replay leaves the same amplitudes
+    for (size_t i = 0; i < n && !rc; i += 2 * kRunGates) {
+        const size_t k = std::min<size_t>(n - i, 2 * kRunGates);
+        rc = sv->dtype == QK_C128 ? launch_ops<double2>((double2 *)sv->d, sv->n, ops.data() + i, k, cs)
+                                  : launch_ops<float2>((float2 *)sv->d, sv->n, ops.data() + i, k, cs);
+    }
     cudaGraph_t g = nullptr;
     e = cudaStreamEndCapture(cs, &g);
     cudaStreamDestroy(cs);
