@@ -408,7 +408,7 @@ struct Builder {
             return 16 + k * (2 * c + (sizeof(double) << (T - r)));
         }
         case OP_SWAP2: return 64;
-        default: return 24 + c;
+        default: return 24 + 4 * c;   // (a condition's share of the tables)
         }
     }
 
@@ -834,12 +834,30 @@ struct Builder {
         for (const auto &c : cond) simple = simple && c.first != kNoQubit && (c.first & kSignFlag);
         const int s = slot(P, op.q[0]);
         if (!simple) {
-            if (op.aux & kRightPhase) cond.push_back({kNoQubit, cget(op.m, 1)});   // part of the pending factor
-            for (size_t c0 = 0; c0 < cond.size(); c0 += 8) {
+            // tables of the factors' products, the right phase and factors
+            // without a condition in the first
+            cl all = (op.aux & kRightPhase) ? cl(cget(op.m, 1)) : cl(1);
+            std::vector<std::pair<uint8_t, cd>> bits;
+            for (const auto &c : cond) {
+                if (c.first == kNoQubit) all *= cl(c.second);
+                else bits.push_back({(uint8_t)(c.first & ~kSignFlag), c.second});
+            }
+            for (size_t c0 = 0; c0 < bits.size() || c0 == 0; c0 += 8) {
                 TOp &t = step(TOP_LAM);
-                for (size_t i = c0; i < std::min(c0 + 8, cond.size()); ++i) t.bits[t.nbits++] = cond[i].first;
-                for (size_t i = c0; i < std::min(c0 + 8, cond.size()); ++i)
-                    if (cond[i].first == kNoQubit || !(cond[i].first & kSignFlag)) push(cond[i].second);
+                t.nbits = (uint8_t)std::min<size_t>(8, bits.size() - c0);
+                for (int i = 0; i < t.nbits; ++i) {
+                    const uint8_t c = bits[c0 + i].first;
+                    t.bits[i] = (c & kOuterFlag) ? (uint8_t)(kOuterFlag | P.outer[c & 0x3F]) : c;
+                }
+                const int nb = t.nbits;
+                for (int i0 = 0; i0 == 0 || i0 < nb; i0 += 4)
+                    for (int i = 0; i < 16; ++i) {
+                        if (i >> std::min(4, nb - i0) && i0) break;   // (the first table is full)
+                        cl f = c0 == 0 && i0 == 0 ? all : cl(1);
+                        for (int k = 0; k < std::min(4, nb - i0); ++k)
+                            if ((i >> k) & 1) f *= cl(bits[c0 + i0 + k].second);
+                        push(to_double(f));
+                    }
             }
         } else if ((layer.k >> s) & 1) {
             flush();

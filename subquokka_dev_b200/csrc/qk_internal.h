@@ -113,8 +113,10 @@ enum TOpKind : uint8_t {
     TOP_LAYER = 14,
     TOP_LCX = 15,   // label step: tile bit a ^= qubit code b (a CX whose swap the next TOP_REMAP performs)
     TOP_PH2 = 16,   // 16 + slot_pair(a, b): amplitude *= coef[0] where slots a and b are 1
-    TOP_LAM = 28,   // pending factor of the next TOP_LAYER: for each of the nbits <= 8 condition codes
-                    // in bits whose qubit is 1 times the next coef, or -1 for a code with kSignFlag
+    TOP_LAM = 28,   // pending factor of the next TOP_LAYER *= the entries of two tables: coef[i], i the
+                    // bits of the first four condition codes in bits, and (nbits > 4)
+                    // coef[16 + j], j those of the others.  A code: a tile bit, or kOuterFlag | bit of
+                    // the tile number
     TOP_SCALE = 29, // amplitude *= coef[0] (b = 1: complex, 0: its real part)
 };
 constexpr uint8_t kLayerWords = 0x20, kLayerSigns = 0x40, kLayerPending = 0x80;   // TOP_LAYER, high half of b

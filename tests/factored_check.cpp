@@ -114,17 +114,6 @@ void emulate(const HostPlan &hp, State &psi, State *lam, std::vector<double> &g)
                     if (op.coef + k >= (uint32_t)d.ncoef) std::exit(2);
                     return cd(hp.coef[2 * i], hp.coef[2 * i + 1]);
                 };
-                auto conditions = [&](int th, int c0) {
-                    cd f = 1;
-                    for (int i = 0; i < op.nbits; ++i) {
-                        const uint8_t code = op.bits[i];
-                        const bool sign = code != qk::kNoQubit && (code & qk::kSignFlag);
-                        const bool b = t.bit(sign ? (uint8_t)(code & ~qk::kSignFlag) : code, th);
-                        const cd c = sign ? cd(-1) : coef(c0++);
-                        if (b) f *= c;
-                    }
-                    return f;
-                };
                 if (op.kind == qk::TOP_LAYER) {
                     uint16_t w[5] = {0};
                     uint32_t u[5] = {0};
@@ -189,7 +178,16 @@ void emulate(const HostPlan &hp, State &psi, State *lam, std::vector<double> &g)
                                     for (int k = 0; k < NT * R; ++k)
                                         if (((k >> a) & 1) && ((k >> b) & 1)) x[k] *= coef(0);
                 } else if (op.kind == qk::TOP_LAM) {
-                    for (int th = 0; th < NT; ++th) pend[th] *= conditions(th, 0);
+                    for (int th = 0; th < NT; ++th) {
+                        int idx = 0;
+                        for (int i = 0; i < op.nbits; ++i) {
+                            const uint8_t c = op.bits[i];
+                            const bool b = (c & qk::kOuterFlag) ? (o >> (c & 31)) & 1 : t.bit(c, th);
+                            idx |= (int)b << i;
+                        }
+                        pend[th] *= coef(idx & 15);
+                        if (op.nbits > 4) pend[th] *= coef(16 + (idx >> 4));
+                    }
                 } else if (op.kind == qk::TOP_LCX) {
                     dirty = true;
                     for (int th = 0; th < NT; ++th)
