@@ -48,9 +48,8 @@ __global__ void __launch_bounds__(MAXT, MINB) k_fpass(C *__restrict__ s, C *__re
         return pass_off(slot_deposit<LOG2R>(tid, op.y, op.z), d);
     };
     const uint64_t g_first = lane_offset(0), g_last = lane_offset(d.last);
-    const int my_bit = outer_bit(d);
     for (uint32_t o = blockIdx.x; o < ntiles; o += gridDim.x) {
-        const uint64_t base = tile_base(o, my_bit, d);
+        const uint64_t base = pass_base(o, d);
         C v[R], w[NS == 2 ? R : 1];
         C *a[R];
         slot_addresses<LOG2R>(s + (base | g_first), d.fpos, a);

@@ -40,22 +40,6 @@ __device__ __forceinline__ void slot_addresses(C *p, const int32_t (&pos)[kPassM
         for (int k = 0; k < (1 << s); ++k) a[k | (1 << s)] = a[k] + (1ull << pos[s]);
 }
 
-// State offset of tile number o.  Lane k of a warp holds the state bit of the
-// number's bit k (outer_bit) and contributes it; a loop over the bits, as in
-// pass_base, took about 80 instructions a tile.
-__device__ __forceinline__ int outer_bit(const PassDesc &d) {
-    int q = threadIdx.x & 31;   // the q-th state bit that is no tile bit
-#pragma unroll 1
-    for (int k = 0; k < d.T; ++k) q += d.bpos[k] <= q;
-    return q < 63 ? q : 63;
-}
-__device__ __forceinline__ uint64_t tile_base(uint32_t o, int my_bit, const PassDesc &d) {
-    if (blockDim.x < 32) return pass_base(o, d);
-    const uint64_t mine = (uint64_t)((o >> (threadIdx.x & 31)) & 1u) << my_bit;
-    return (uint64_t)__reduce_or_sync(0xffffffffu, (uint32_t)(mine >> 32)) << 32 |
-           __reduce_or_sync(0xffffffffu, (uint32_t)mine);
-}
-
 // a * s + c, both components (complex64: one packed instruction, the same
 // roundings as two).
 __device__ __forceinline__ double2 axpy(double s, double2 a, double2 c) {
