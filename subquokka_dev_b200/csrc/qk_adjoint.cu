@@ -133,8 +133,11 @@ struct PauliTile {
 // 64-bit words with a bit a term, of which only the tile's is made anew for a
 // tile (a lane a term).  With the parities taken term by term, POPC bound the
 // kernel (27 qubits, 53 terms: 7.6 ms).  Groups of one X string, the common
-// case, run ahead of the others in a loop of their own.
-template <typename C>
+// case, have a loop of their own.
+// ROUND: out's sum is rounded to C after every group, the groups of several
+// terms first, as by a sweep a group (complex64 gradients keep their values
+// so: with one rounding a tile they changed by 6e-8); acc is not used.
+template <typename C, bool ROUND>
 __global__ void __launch_bounds__(kRedThreads, 2) k_pauli_tile(C *__restrict__ out, const C *__restrict__ psi, uint64_t ntiles,
                                                             const __grid_constant__ PauliTile t, int accumulate,
                                                             double *acc) {
@@ -212,23 +215,26 @@ __global__ void __launch_bounds__(kRedThreads, 2) k_pauli_tile(C *__restrict__ o
         }
         double re[E], im[E];
 #pragma unroll
-        for (int u = 0; u < E; ++u) re[u] = im[u] = 0;
+        for (int u = 0; u < E; ++u) {
+            re[u] = im[u] = 0;
+            if (ROUND && accumulate && tid + u * NT < N) {
+                const C b = out[here | off[u]];
+                re[u] = b.x;
+                im[u] = b.y;
+            }
+        }
+        auto rounded = [&](int u) {
+            if constexpr (ROUND) {
+                const C b = mk<C>(re[u], im[u]);
+                re[u] = b.x;
+                im[u] = b.y;
+            }
+        };
         // += (fr + i fi) b, the group's factor at the element
         auto add = [&](int u, const C b, double fr, double fi) {
             re[u] += fr * (double)b.x - fi * (double)b.y;
             im[u] += fr * (double)b.y + fi * (double)b.x;
         };
-#pragma unroll 4
-        for (int g = 0; g < t.nsimple; ++g) {
-            const double c = t.scoef[g];
-            const uint32_t xp = t.splace[g];
-#pragma unroll
-            for (int u = 0; u < E; ++u) {
-                const C b = *reinterpret_cast<const C *>(smem_raw + (place[u] ^ xp));
-                re[u] += c * (double)b.x;
-                im[u] += c * (double)b.y;
-            }
-        }
         for (int g = 0; g < t.ngroups; ++g) {
             const int t0 = t.term0[g], t1 = t.term0[g + 1];
             const uint32_t xp = t.xplace[g];
@@ -247,8 +253,22 @@ __global__ void __launch_bounds__(kRedThreads, 2) k_pauli_tile(C *__restrict__ o
                 }
             }
 #pragma unroll
-            for (int u = 0; u < E; ++u)
+            for (int u = 0; u < E; ++u) {
                 add(u, *reinterpret_cast<const C *>(smem_raw + (place[u] ^ xp)), fr[u], fi[u]);
+                rounded(u);
+            }
+        }
+#pragma unroll 4
+        for (int g = 0; g < t.nsimple; ++g) {
+            const double c = t.scoef[g];
+            const uint32_t xp = t.splace[g];
+#pragma unroll
+            for (int u = 0; u < E; ++u) {
+                const C b = *reinterpret_cast<const C *>(smem_raw + (place[u] ^ xp));
+                re[u] += c * (double)b.x;
+                im[u] += c * (double)b.y;
+                rounded(u);
+            }
         }
 #pragma unroll
         for (int u = 0; u < E; ++u)
@@ -256,7 +276,7 @@ __global__ void __launch_bounds__(kRedThreads, 2) k_pauli_tile(C *__restrict__ o
                 sum += (double)v[u].x * re[u] + (double)v[u].y * im[u];
                 if (out) {
                     C *p = out + (here | off[u]);
-                    if (accumulate) {
+                    if (!ROUND && accumulate) {
                         re[u] += p->x;
                         im[u] += p->y;
                     }
@@ -372,16 +392,8 @@ static_assert(1 << (kPauliTileBits - kTileSlots) == kRedThreads, "elements a thr
 
 // The groups whose X masks fit a tile, cut into tiles; the others stay in
 // `flat` (one sweep each).
-//
-// A complex64 H psi is written group by group, each sum rounded to 24 bits,
-// as the gradients of complex64 sweeps have been computed: with one rounding
-// a tile they changed by 6e-8.
-static void tile_groups(const std::vector<PauliGroup> &groups, int n, int dtype, bool apply, std::vector<PauliTile> &tiles,
+static void tile_groups(const std::vector<PauliGroup> &groups, int n, int dtype, std::vector<PauliTile> &tiles,
                         std::vector<PauliGroup> &flat) {
-    if (apply && dtype == QK_C64) {
-        flat = groups;
-        return;
-    }
     const int T = std::min(n, kPauliTileBits), L = std::min(T, dtype == QK_C128 ? 3 : 4);   // 128-byte runs
     const uint64_t low = (1ull << L) - 1;
     std::vector<const PauliGroup *> left;
@@ -436,7 +448,7 @@ static void tile_groups(const std::vector<PauliGroup> &groups, int n, int dtype,
 static size_t pauli_sweeps(const std::vector<PauliGroup> &groups, int n, int dtype) {
     std::vector<PauliTile> tiles;
     std::vector<PauliGroup> flat;
-    tile_groups(groups, n, dtype, true, tiles, flat);
+    tile_groups(groups, n, dtype, tiles, flat);
     return tiles.size() + flat.size();
 }
 
@@ -450,17 +462,20 @@ static int pauli_sum_t(C *out, const C *psi, int n, const std::vector<PauliGroup
     }
     std::vector<PauliTile> tiles;
     std::vector<PauliGroup> flat;
-    tile_groups(groups, n, sizeof(C) == sizeof(double2) ? QK_C128 : QK_C64, out != nullptr, tiles, flat);
+    tile_groups(groups, n, sizeof(C) == sizeof(double2) ? QK_C128 : QK_C64, tiles, flat);
+    constexpr bool c64 = sizeof(C) == sizeof(float2);
+    const bool round = c64 && out, dot = out && acc && (round || !flat.empty());   // dot: <H> from all of H psi
+    const auto kernel = round ? k_pauli_tile<C, c64> : k_pauli_tile<C, false>;
     int done = 0;
     for (const PauliTile &t : tiles) {
         const unsigned threads = std::min(kRedThreads, std::max(32, (1 << t.d.T) >> kTileSlots));
         const size_t smem = sizeof(C) << t.d.T;
         int mb = 0;
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&mb, k_pauli_tile<C>, (int)threads, smem);
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&mb, kernel, (int)threads, smem);
         if (e != cudaSuccess || mb < 1) mb = 1;
         const uint64_t ntiles = namp >> t.d.T;
         const unsigned grid = (unsigned)std::min<uint64_t>(ntiles, (uint64_t)device_sms() * mb);
-        k_pauli_tile<C><<<grid, threads, smem, st>>>(out, psi, ntiles, t, done++ > 0, acc);
+        kernel<<<grid, threads, smem, st>>>(out, psi, ntiles, t, done++ > 0, dot ? nullptr : acc);
         e = cudaGetLastError();
         if (e != cudaSuccess) return cuda_err(e, "k_pauli_tile");
     }
@@ -468,12 +483,7 @@ static int pauli_sum_t(C *out, const C *psi, int n, const std::vector<PauliGroup
         if (out) k_pauli_apply<C><<<red_grid(namp), kRedThreads, 0, st>>>(out, psi, namp, g, done++ > 0);
         else k_pauli_expval<C><<<red_grid(namp), kRedThreads, 0, st>>>(psi, namp, g, acc);
     }
-    if (out && acc && !flat.empty()) {
-        // <H> from all of H psi
-        cudaError_t e = cudaMemsetAsync(acc, 0, sizeof(double), st);
-        if (e != cudaSuccess) return cuda_err(e, "clear accumulator");
-        k_dot_re<C><<<red_grid(namp), kRedThreads, 0, st>>>(psi, out, namp, acc);
-    }
+    if (dot) k_dot_re<C><<<red_grid(namp), kRedThreads, 0, st>>>(psi, out, namp, acc);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? QK_OK : cuda_err(e, "k_pauli");
 }
