@@ -40,8 +40,8 @@ template <typename C> struct BatchEntry {
 };
 
 // One persistent launch over the k-th pass of every circuit.
-template <typename C, int R, int NS>
-__global__ void __launch_bounds__(pass_max_threads<C, R, NS>()) k_pass_batch(const BatchEntry<C> *__restrict__ tab,
+template <typename C, int R, int NS, int MAXT, int MINB>
+__global__ void __launch_bounds__(MAXT, MINB) k_pass_batch(const BatchEntry<C> *__restrict__ tab,
                                                                             int nent, uint64_t total, uint64_t chunk) {
     constexpr int LOG2R = R == 2 ? 1 : R == 4 ? 2 : R == 8 ? 3 : R == 16 ? 4 : 5;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -379,22 +379,32 @@ static int build_tables(qk_batch *b) {
     return QK_OK;
 }
 
-template <typename C, int R, int NS>
-static int launch_batch_step(const qk_batch::Step &s, cudaStream_t st) {
+template <typename C, int R, int NS, int MAXT, int MINB>
+static int launch_batch_k(const qk_batch::Step &s, cudaStream_t st) {
     static std::atomic<uint64_t> smem_done{0};
-    const cudaError_t ea = smem_limit_once(smem_done, (const void *)k_pass_batch<C, R, NS>, 220 << 10);
+    const cudaError_t ea = smem_limit_once(smem_done, (const void *)k_pass_batch<C, R, NS, MAXT, MINB>, 220 << 10);
     if (ea != cudaSuccess) return cuda_err(ea, "cudaFuncSetAttribute(k_pass_batch)");
     const int sms = device_sms();
     const unsigned threads = (1u << s.T) / R;
     int mb = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&mb, k_pass_batch<C, R, NS>, (int)threads, s.smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&mb, k_pass_batch<C, R, NS, MAXT, MINB>, (int)threads, s.smem);
     if (mb < 1) mb = 1;
     const uint64_t ctas = std::min<uint64_t>(s.total, (uint64_t)sms * mb);
     const uint64_t chunk = (s.total + ctas - 1) / ctas;
     const unsigned grid = (unsigned)((s.total + chunk - 1) / chunk);
-    k_pass_batch<C, R, NS><<<grid, threads, s.smem, st>>>((const BatchEntry<C> *)s.tab, s.nent, s.total, chunk);
+    k_pass_batch<C, R, NS, MAXT, MINB><<<grid, threads, s.smem, st>>>((const BatchEntry<C> *)s.tab, s.nent, s.total, chunk);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? QK_OK : cuda_err(e, "k_pass_batch launch");
+}
+
+template <typename C, int R, int NS>
+static int launch_batch_step(const qk_batch::Step &s, cudaStream_t st) {
+    // complex64 steps on the default tiles (128 threads): held to 80 registers
+    // a thread, six CTAs an SM (some spills: 40 circuits of 14-20 qubits 8.8 ms
+    // against 9.2 with five and 9.7 unbounded, 127 registers)
+    if constexpr (sizeof(C) == sizeof(float2) && ((R == 8 && NS == 2) || (R == 16 && NS == 1)))
+        if ((1u << s.T) / R <= 128) return launch_batch_k<C, R, NS, 128, 6>(s, st);
+    return launch_batch_k<C, R, NS, pass_max_threads<C, R, NS>(), 1>(s, st);
 }
 
 template <typename C>

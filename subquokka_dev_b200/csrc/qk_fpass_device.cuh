@@ -17,18 +17,6 @@
 
 namespace qk {
 
-// tid with a zero bit inserted at each of the slots' tile bits (ascending).
-template <int LOG2R>
-__device__ __forceinline__ uint32_t slot_deposit(uint32_t tid, uint32_t bits4, uint32_t bit5) {
-    uint32_t x = tid;
-#pragma unroll
-    for (int s = 0; s < LOG2R; ++s) {
-        const uint32_t hi = ~0u << ((s < 4 ? bits4 >> (8 * (s & 3)) : bit5) & 31);
-        x += x & hi;
-    }
-    return x;
-}
-
 // Addresses of a thread's register elements: the state at p, slot s the
 // state bit pos[s].
 template <int LOG2R, typename C>

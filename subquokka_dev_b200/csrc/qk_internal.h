@@ -87,7 +87,8 @@ constexpr int kPassMaxBits = 14;
 constexpr int kPassMaxReg = 5;
 
 enum TOpKind : uint8_t {
-    TOP_REMAP = 0,  // re-distribute the tile: register slot s <- tile bit bits[s]
+    TOP_REMAP = 0,  // re-distribute the tile: register slot s <- tile bit bits[s] (bits[4..7]: the
+                    // same ascending)
     TOP_G1 = 1,     // dense 2x2 on register slot a; coef -> 4 complex
     TOP_G2 = 2,     // dense 4x4 on register slots a < b (index bit0 = a); coef -> 16 complex
     TOP_DIAG = 3,   // amplitude *= coef[bit(a) + 2 bit(b)]; a, b are qubit codes

@@ -30,7 +30,7 @@ namespace qk {
 // gradient accumulators of the pass live in shared memory and are added to
 // ggrad[gparams[grad0 + i]] once per CTA.
 template <typename C, int R, int NS, bool NARROW, bool XOPS>
-__global__ void __launch_bounds__(NARROW ? 128 : pass_max_threads<C, R, NS>(), NARROW ? 3 : 1) k_pass(C *__restrict__ s, C *__restrict__ s2, uint64_t ntiles,
+__global__ void __launch_bounds__(NARROW ? 128 : pass_max_threads<C, R, NS>(), NARROW ? pass_narrow_ctas<C, R, NS>() : 1) k_pass(C *__restrict__ s, C *__restrict__ s2, uint64_t ntiles,
                                                        const __grid_constant__ PassDesc d, const TOp *__restrict__ gprog,
                                                        const C *__restrict__ gcoef, const int32_t *__restrict__ gparams,
                                                        double *__restrict__ ggrad, int nbuf) {
@@ -179,7 +179,7 @@ static int launch_pass_r(const PassArgs<C> &a, int n, const PassDesc &d, cudaStr
     // specialises them; the others on one without that code, whose register
     // allocation it would otherwise change (the 30-qubit random circuit and
     // HEA forward passes, which have neither, 1-2.5 % slower with it)
-    if constexpr (pass_narrow_ok<C, R, NS>())
+    if constexpr (pass_narrow_ctas<C, R, NS>() > 0)
         if (!d.perm && threads <= 128)
             return d.xops ? launch_pass_k<C, R, NS, true, true>(a, n, d, threads, st)
                           : launch_pass_k<C, R, NS, true, false>(a, n, d, threads, st);

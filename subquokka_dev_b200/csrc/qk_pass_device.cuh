@@ -35,14 +35,15 @@ constexpr int pass_max_threads() {
     return sizeof(C) * R * NS >= 256 ? 256 : kPassThreads;
 }
 
-// The complex128 single-state pass with 16 amplitudes a thread on its
-// default 2048-amplitude tiles has 128 threads; a second instance of it is
-// bounded to 128 threads and three CTAs an SM: 168 registers instead of 241,
-// 12 warps an SM instead of 8 (0.645 -> 0.600 s on the 30-qubit random
-// circuit).
+// Instances bounded to 128 threads (2048-amplitude tiles, 16 amplitudes a
+// thread) hold this many CTAs an SM; 0: there is none.  complex128, one state:
+// three, 168 registers instead of 241, 12 warps an SM instead of 8 (0.645 ->
+// 0.600 s on the 30-qubit random circuit).  complex64, two states: three, 168
+// registers instead of 254, and one state: five, 96 instead of 128 (26-qubit
+// HEA sweep 100.5 -> 89.9 ms; six CTAs of one state 90.4).
 template <typename C, int R, int NS>
-constexpr bool pass_narrow_ok() {
-    return sizeof(C) == 16 && R == 16 && NS == 1;
+constexpr int pass_narrow_ctas() {
+    return R != 16 ? 0 : sizeof(C) == 16 ? (NS == 1 ? 3 : 0) : NS == 1 ? 5 : 3;
 }
 
 // Scatter the low bits of v into the set bits of mask, lowest first.
@@ -55,6 +56,19 @@ __device__ __forceinline__ uint32_t deposit_bits(uint32_t v, uint32_t mask) {
         mask ^= low;
     }
     return r;
+}
+
+// tid with a zero bit inserted at each of the slots' tile bits (ascending,
+// bytes of bits4, the fifth bit5).
+template <int LOG2R>
+__device__ __forceinline__ uint32_t slot_deposit(uint32_t tid, uint32_t bits4, uint32_t bit5) {
+    uint32_t x = tid;
+#pragma unroll
+    for (int s = 0; s < LOG2R; ++s) {
+        const uint32_t hi = ~0u << ((s < 4 ? bits4 >> (8 * (s & 3)) : bit5) & 31);
+        x += x & hi;
+    }
+    return x;
 }
 
 template <int LOG2R>
@@ -506,14 +520,12 @@ __device__ __forceinline__ void run_program(C *tl, C *tw, uint64_t base, const P
                 }
             }
             __syncthreads();
-            uint32_t regmask = 0;
 #pragma unroll
             for (int q = 0; q < LOG2R; ++q) {
                 bm[q] = 1u << op.bits[q];
                 sb[q] = swz<C>(bm[q]);
-                regmask |= bm[q];
             }
-            tb = deposit_bits(tid, (N - 1) & ~regmask);
+            tb = slot_deposit<LOG2R>(tid, op.bits[4] | op.bits[5] << 8 | op.bits[6] << 16 | (uint32_t)op.bits[7] << 24, 0);
             stb = swz<C>(tb);
 #pragma unroll
             for (int kk = 0; kk < R; ++kk) {

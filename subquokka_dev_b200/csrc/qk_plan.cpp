@@ -230,7 +230,8 @@ struct PassBuilder {
             std::memset(&t, 0, sizeof t);
             t.kind = TOP_REMAP;
             t.nbits = (uint8_t)r;
-            for (int s = 0; s < r; ++s) t.bits[s] = (uint8_t)Q[s];
+            for (int s = 0; s < r; ++s) t.bits[s] = t.bits[4 + s] = (uint8_t)Q[s];
+            std::sort(t.bits + 4, t.bits + 4 + r);   // (r <= 4)
             plan.ops.push_back(t);
             ++plan.nremaps;
             mapped = true;
