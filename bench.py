@@ -240,6 +240,23 @@ def measured_peak_hbm():
 # ---------------------------------------------------------------------------
 # our arm
 # ---------------------------------------------------------------------------
+def gate_launches(circ) -> int:
+    """Kernel launches of the per-gate path: runs of two or more diagonal gates
+    (at most 32, within windows of 64 gates) share one (csrc/qk_engine.cu launch_ops)."""
+    diagonal = {4, 5, 8, 12, 13}   # Z, P, RZ, CP, RZZ
+    count = 0
+    kinds = [g.kind in diagonal for g in circ.gate_list()]
+    for w in range(0, len(kinds), 64):
+        run = 0
+        for d in kinds[w:w + 64]:
+            if d and 0 < run < 32:
+                run += 1
+                continue
+            count += 1
+            run = 1 if d else 0
+    return count
+
+
 def kernel_class(g):
     """Name of the kernel a gate launches (see csrc/qk_engine.cu launch_op)."""
     if g.kind == 9:

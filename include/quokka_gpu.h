@@ -203,7 +203,9 @@ int qk_sv_release_workspace(qk_sv *sv);
 
 /* ---- the hot path ------------------------------------------------------ */
 
-/* Per-gate path: apply gates[0..n) in order, one state sweep per gate.
+/* Per-gate path: apply gates[0..n) in order, one state sweep per gate; runs of
+ * consecutive diagonal gates (Z, P, RZ, CP, RZZ, diagonal U2) share a sweep
+ * that gives each amplitude their factors in order.
  * Replaces MEM_Runner::run(std::vector<Gate*>&) (src/MEM_Runner.cpp:101-134).
  * Asynchronous on the state's stream. */
 int qk_apply_gates(qk_sv *sv, const qk_gate *gates, size_t n);
@@ -247,10 +249,11 @@ int qk_apply_gates_timed(qk_sv *sv, const qk_gate *gates, size_t n, float *gate_
 /* Options of a fused plan; zero fields take the defaults. */
 typedef struct qk_plan_opts {
     int32_t dtype;        /* qk_dtype of the states the plan runs on        */
-    int32_t tile_bits;    /* qubits per shared-memory tile (default 11; at
-                             most 14)                                       */
-    int32_t reg_bits;     /* qubits held in registers per thread (default 4;
-                             at most 5)                                     */
+    int32_t tile_bits;    /* qubits per shared-memory tile (at most 14;
+                             default 11, 10 / 12 for factored complex128 /
+                             complex64 programs: see qk_plan_create)        */
+    int32_t reg_bits;     /* qubits held in registers per thread (at most 4;
+                             default 4, 5 for factored complex64 programs)  */
     int32_t fuse_width;   /* 0: register passes.  5 or 6: gates fused into
                              dense unitaries on at most that many qubits
                              (FP64 on the host, padded to 6 qubits), each
@@ -274,7 +277,9 @@ typedef struct qk_plan qk_plan;
  * for any circuit, with no VSWAP: a tile's qubits need not be contiguous.
  * VSWAP gates of the list rename qubits instead of moving amplitudes, and so
  * do SWAP gates when that gives fewer passes; a final permutation restores
- * the layout. */
+ * the layout.  Circuits whose one-qubit gates are unitary and whose two-qubit
+ * gates are diagonal, CNOT or SWAP run factored programs (a unitary as two
+ * phases and a rotation, CNOT and SWAP as labels), others dense ones. */
 int qk_plan_create(const qk_gate *gates, size_t n, int nqubits, const qk_plan_opts *opts, qk_plan **out);
 /* The plan of a subcircuit file that qk_apply_groups runs: the gates of all
  * groups fused as one list, VSWAPs as renamings of the qubits after them.
@@ -307,8 +312,9 @@ typedef struct qk_pauli_term {
     uint64_t z_mask;
 } qk_pauli_term;
 
-/* <psi| H |psi> for H = sum of the terms (one state sweep per distinct
- * x_mask; the state is not modified). */
+/* <psi| H |psi> for H = sum of the terms (the state is not modified).  One
+ * state sweep takes all terms whose X masks lie in the bits of a tile: the
+ * lowest few and about seven others; a wider mask has a sweep of its own. */
 int qk_expval_pauli(qk_sv *sv, const qk_pauli_term *terms, size_t nterms, double *out);
 
 /* Adjoint gradient of <H> after gates[0..ngates) applied to the state in sv.

@@ -1,7 +1,8 @@
 // State handles, kernel dispatch and the hot-path entry points of the C ABI.
 //
 // qk_apply_gates is the GPU counterpart of MEM_Runner::run(vector<Gate*>&)
-// (src/MEM_Runner.cpp:101-134): gates in order, one state sweep each.
+// (src/MEM_Runner.cpp:101-134): gates in order, one state sweep each, runs of
+// diagonal gates one together.
 // qk_apply_groups is the counterpart of MEM_Runner::run(vector<vector<Gate*>>&)
 // (src/MEM_Runner.cpp:136-185): every gate group becomes one shared-memory
 // tile pass over the state.

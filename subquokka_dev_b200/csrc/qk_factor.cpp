@@ -852,7 +852,8 @@ struct Builder {
                 const int nb = t.nbits;
                 for (int i0 = 0; i0 == 0 || i0 < nb; i0 += 4)
                     for (int i = 0; i < 16; ++i) {
-                        if (i >> std::min(4, nb - i0) && i0) break;   // (the first table is full)
+                        // (full where a second one follows)
+                        if (i >> std::min(4, nb - i0) && (i0 || nb <= 4)) break;
                         cl f = c0 == 0 && i0 == 0 ? all : cl(1);
                         for (int k = 0; k < std::min(4, nb - i0); ++k)
                             if ((i >> k) & 1) f *= cl(bits[c0 + i0 + k].second);
