@@ -240,23 +240,6 @@ def measured_peak_hbm():
 # ---------------------------------------------------------------------------
 # our arm
 # ---------------------------------------------------------------------------
-def gate_launches(circ) -> int:
-    """Kernel launches of the per-gate path: runs of two or more diagonal gates
-    (at most 32, within windows of 64 gates) share one (csrc/qk_engine.cu launch_ops)."""
-    diagonal = {4, 5, 8, 12, 13}   # Z, P, RZ, CP, RZZ
-    count = 0
-    kinds = [g.kind in diagonal for g in circ.gate_list()]
-    for w in range(0, len(kinds), 64):
-        run = 0
-        for d in kinds[w:w + 64]:
-            if d and 0 < run < 32:
-                run += 1
-                continue
-            count += 1
-            run = 1 if d else 0
-    return count
-
-
 def kernel_class(g):
     """Name of the kernel a gate launches (see csrc/qk_engine.cu launch_op)."""
     if g.kind == 9:
@@ -740,7 +723,7 @@ def our_arm(args, rank, world):
                 "kernel_share": {k: v / tot for k, v in sorted(shares.items())},
                 "kernel_gbs": {k: (2 * S if k.startswith("k_dense1") else S // 2) / (statistics.mean(v) / 1e3) / 1e9
                                for k, v in per_kernel.items()}}
-    launches = args.steps * (gate_launches(circ) + 1)
+    launches = args.steps * (circ.ngates + 1)
     # the fused forms and the other workloads are single-GPU measurements:
     # a run on N > 1 GPUs (replicas of the timed step) skips them and runs
     # the two multi-GPU legs instead, so that it holds the GPUs briefly
