@@ -515,7 +515,7 @@ struct Builder {
         std::vector<int> B;      // empty: a permutation pass, take[0]
     };
     std::vector<Part> parts = {};
-    void partition() {
+    int partition() {
         make_lite();
         std::vector<size_t> pending(ops.size()), rest;
         for (size_t i = 0; i < ops.size(); ++i) pending[i] = i;
@@ -536,6 +536,8 @@ struct Builder {
                 (ok ? p.take : rest).push_back(i);
                 return true;
             });
+            if (p.take.empty())
+                return fail(QK_ERR_ARG, "tile_bits %d: an operation needs %d tile qubits", T, lite[pending[0]].nb);
             defer(p.take, rest);
             for (int q = 0; q < n && nB < T; ++q)
                 if (!inB[q]) inB[q] = 1, ++nB;
@@ -544,6 +546,7 @@ struct Builder {
             parts.push_back(std::move(p));
             pending.swap(rest);
         }
+        return QK_OK;
     }
 
     int compile_parts() {
@@ -1063,13 +1066,16 @@ int build_best(const std::vector<std::vector<Op>> &lists, const std::vector<cl> 
         if (variant % 2) asap_order(c.ops, n);
         HostPlan hp = empty;
         Builder b{c.ops, n, o.f_tile_bits, o.f_reg_bits, L, hp, o, variant >= 2, scale[list], scaled[list] != 0};
-        b.partition();
+        const int rc = b.partition();
         c.parts.swap(b.parts);
-        return (int)QK_OK;
+        return rc;
     };
     // (a thread costs some 30 us to start, a candidate of a few hundred ops more)
     const bool threads = o.threads && lists[0].size() >= 100;
-    for (size_t k = 0; k < all.size() && !threads; ++k) candidate(k);
+    for (size_t k = 0; k < all.size() && !threads; ++k) {
+        int rc = candidate(k);
+        if (rc) return rc;
+    }
     if (threads) {
         int rc = run_tasks(all.size(), candidate);
         if (rc) return rc;

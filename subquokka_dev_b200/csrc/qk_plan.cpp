@@ -543,6 +543,8 @@ struct PassBuilder {
                     rest.push_back(i);
                 }
             }
+            if (take.empty())
+                return fail(QK_ERR_ARG, "tile_bits %d: an operation needs %d tile qubits", T, op_reg_count(ops[pending[0]]));
             fill(B);
             int rc = compile(take, B);
             if (rc) return rc;

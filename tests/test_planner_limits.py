@@ -1,0 +1,40 @@
+"""Planner calls that have no plan end with an error, and soon (CPU)."""
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+from subquokka_dev_b200 import Circuit, Plan, make_gate
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.mark.parametrize("dtype", ["c128", "c64"])
+@pytest.mark.parametrize("gates", [
+    'make_gate("RY", [0], 0.3), make_gate("SWAP", [0, 2])',                                # factored programs
+    'make_gate("RY", [0], 0.3), make_gate("U2", [0, 2], 0.0, np.linalg.qr(m)[0])',         # general programs
+])
+def test_two_tile_qubits_in_a_one_qubit_tile_is_an_error(dtype, gates):
+    # in a child with a limit: a planner that makes no progress does not return
+    code = f"""
+import resource
+resource.setrlimit(resource.RLIMIT_AS, (8 << 30, 8 << 30))
+import numpy as np
+from subquokka_dev_b200 import Circuit, Plan, make_gate
+m = np.random.default_rng(1).standard_normal((4, 4))
+try:
+    Plan(Circuit([{gates}]), 3, "{dtype}", tile_bits=1, reg_bits=1)
+except Exception as e:
+    print(type(e).__name__, e)
+"""
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0 and "QK_ERR_ARG" in r.stdout and "needs 2 tile qubits" in r.stdout, r.stdout + r.stderr
+
+
+def test_one_qubit_tiles_take_what_needs_one():
+    cnot = np.eye(4)[[0, 1, 3, 2]]
+    c = Circuit([make_gate("RY", [0], 0.3), make_gate("CP", [0, 1], 0.4), make_gate("U2", [0, 2], 0.0, cnot)])
+    for dtype in ("c128", "c64"):
+        assert Plan(c, 3, dtype, tile_bits=1, reg_bits=1).stats()[0] >= 1
