@@ -640,7 +640,7 @@ static int adjoint_fused_t(C *psi, int n, int dtype, const qk_gate *gates, size_
                      : plan_forward(g, cnt, n, fo, fwd[sgi]);
     };
     if (ng >= 100) {
-        int rc = run_tasks(2 * nseg, plan_one);
+        int rc = run_tasks(2 * nseg, std::ref(plan_one));   // (no allocation for the callable)
         if (rc) return rc;
     }
     for (size_t sgi = 0; sgi < nseg; ++sgi) {

@@ -31,31 +31,32 @@
 namespace qk {
 
 int run_tasks(size_t n, const std::function<int(size_t)> &task) {
-    std::vector<int> rc(n, QK_OK);
-    std::vector<std::string> what(n);
-    std::atomic<size_t> next{0};
-    auto work = [&]() {
-        for (size_t i = next++; i < n; i = next++) {
-            try {
-                rc[i] = task(i);
-            } catch (const std::bad_alloc &) {
-                rc[i] = fail(QK_ERR_OOM, "out of host memory");
+    return no_throw([&]() -> int {
+        std::vector<int> rc(n, QK_OK);
+        std::vector<std::string> what(n);
+        std::atomic<size_t> next{0};
+        auto work = [&]() {
+            for (size_t i = next++; i < n; i = next++) {
+                rc[i] = no_throw([&]() { return task(i); });
+                if (rc[i]) no_throw([&]() { return what[i] = qk_last_error(), QK_OK; });
             }
-            if (rc[i]) what[i] = qk_last_error();
+        };
+        const size_t threads = std::min<size_t>(n, std::max(1u, std::thread::hardware_concurrency()));
+        std::vector<std::thread> pool;
+        pool.reserve(threads);
+        try {
+            for (size_t t = 1; t < threads; ++t) pool.emplace_back(work);
+        } catch (const std::system_error &) {
+            // no more threads: those that run, and this one, take the tasks
+        } catch (const std::bad_alloc &) {
+            // (the same)
         }
-    };
-    std::vector<std::thread> pool;
-    const size_t cores = std::max(1u, std::thread::hardware_concurrency());
-    try {
-        for (size_t t = 1; t < std::min(n, cores); ++t) pool.emplace_back(work);
-    } catch (const std::system_error &) {
-        // no more threads: those that run, and this one, take the tasks
-    }
-    work();
-    for (std::thread &t : pool) t.join();
-    for (size_t i = 0; i < n; ++i)
-        if (rc[i]) return fail(rc[i], "%s", what[i].c_str());
-    return QK_OK;
+        work();
+        for (std::thread &t : pool) t.join();
+        for (size_t i = 0; i < n; ++i)
+            if (rc[i]) return fail(rc[i], "%s", what[i].c_str());
+        return QK_OK;
+    });
 }
 
 // Tile and register bits of factored passes.  complex128: 1024-amplitude
@@ -1113,7 +1114,7 @@ bool plan_is_factored(const qk_gate *gates, size_t ng, int n, const PlanOptions 
     return true;
 }
 
-int plan_forward(const qk_gate *gates, size_t ng, int n, const PlanOptions &o, HostPlan &plan) {
+static int forward(const qk_gate *gates, size_t ng, int n, const PlanOptions &o, HostPlan &plan) {
     int rc = check_options(o, n);
     if (rc) return rc;
     if (!plan_is_factored(gates, ng, n, o, 1)) return build_plan(gates, ng, n, o, plan);
@@ -1141,7 +1142,7 @@ int plan_forward(const qk_gate *gates, size_t ng, int n, const PlanOptions &o, H
     return build_best(lists, scale, scaled, n, o, 1, plan);
 }
 
-int plan_adjoint(const qk_gate *gates, size_t ng, const int32_t *pidx, int n, const PlanOptions &o, HostPlan &plan) {
+static int adjoint(const qk_gate *gates, size_t ng, const int32_t *pidx, int n, const PlanOptions &o, HostPlan &plan) {
     int rc = check_options(o, n);
     if (rc) return rc;
     if (!plan_is_factored(gates, ng, n, o, 2)) return build_adjoint_plan(gates, ng, pidx, n, o, plan);
@@ -1172,6 +1173,14 @@ int plan_adjoint(const qk_gate *gates, size_t ng, const int32_t *pidx, int n, co
     bool scaled;
     factor(ops, n, o.dtype, scale, scaled);
     return build_best({ops}, {scale}, {scaled}, n, o, 2, plan);
+}
+
+int plan_forward(const qk_gate *gates, size_t ng, int n, const PlanOptions &o, HostPlan &plan) {
+    return no_throw([&]() { return forward(gates, ng, n, o, plan); });
+}
+
+int plan_adjoint(const qk_gate *gates, size_t ng, const int32_t *pidx, int n, const PlanOptions &o, HostPlan &plan) {
+    return no_throw([&]() { return adjoint(gates, ng, pidx, n, o, plan); });
 }
 
 int build_group_plan(const qk_gate *gates, const int32_t *sizes, size_t ngroups, int n, const PlanOptions &o,

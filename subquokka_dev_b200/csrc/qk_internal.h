@@ -4,6 +4,8 @@
 #include <cstddef>
 #include <cstdint>
 #include <functional>
+#include <new>
+#include <stdexcept>
 #include <string>
 #include <vector>
 
@@ -41,8 +43,19 @@ struct Op {
 };
 
 // Thread-local error message; returns code so callers can `return fail(...)`.
-int fail(int code, const char *fmt, ...) __attribute__((format(printf, 2, 3)));
+int fail(int code, const char *fmt, ...) noexcept __attribute__((format(printf, 2, 3)));
 void clear_error();
+
+// f()'s code, or QK_ERR_OOM where it runs out of host memory: nothing is
+// thrown past the planners, whose callers are C entry points.
+template <typename F> int no_throw(F &&f) {
+    try {
+        return f();
+    } catch (const std::bad_alloc &) {
+    } catch (const std::length_error &) {
+    }
+    return fail(QK_ERR_OOM, "out of host memory");
+}
 
 // task(0) .. task(n - 1) on up to n host threads, this one among them (all of
 // them on this one where no thread can be had).  Returns the first failing

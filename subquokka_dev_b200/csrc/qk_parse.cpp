@@ -22,13 +22,17 @@ namespace qk {
 
 static thread_local std::string g_last_error;
 
-int fail(int code, const char *fmt, ...) {
+int fail(int code, const char *fmt, ...) noexcept {
     char buf[1024];
     va_list ap;
     va_start(ap, fmt);
     vsnprintf(buf, sizeof buf, fmt, ap);
     va_end(ap);
-    g_last_error = buf;
+    try {
+        g_last_error = buf;
+    } catch (...) {   // no memory for the text
+        g_last_error.clear();
+    }
     return code;
 }
 

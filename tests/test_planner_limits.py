@@ -1,5 +1,6 @@
 """Planner calls that have no plan end with an error, and soon (CPU)."""
 import os
+import shutil
 import subprocess
 import sys
 
@@ -38,3 +39,16 @@ def test_one_qubit_tiles_take_what_needs_one():
     c = Circuit([make_gate("RY", [0], 0.3), make_gate("CP", [0, 1], 0.4), make_gate("U2", [0, 2], 0.0, cnot)])
     for dtype in ("c128", "c64"):
         assert Plan(c, 3, dtype, tile_bits=1, reg_bits=1).stats()[0] >= 1
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="g++ absent")
+def test_failed_allocations_are_errors(tmp_path):
+    csrc = os.path.join(ROOT, "subquokka_dev_b200", "csrc")
+    exe = tmp_path / "alloc_check"
+    cmd = ["g++", "-O1", "-std=c++17", "-I", os.path.join(ROOT, "include"), "-I", csrc, "-I", os.path.join(ROOT, "tests"),
+           os.path.join(ROOT, "tests", "alloc_check.cpp")]
+    cmd += [os.path.join(csrc, f) for f in ("qk_factor.cpp", "qk_plan.cpp", "qk_rewrite.cpp", "qk_parse.cpp", "qk_dense_host.cpp")]
+    build = subprocess.run(cmd + ["-o", str(exe), "-lpthread"], capture_output=True, text=True)
+    assert build.returncode == 0, build.stderr
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout + r.stderr
