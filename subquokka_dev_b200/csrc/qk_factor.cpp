@@ -15,7 +15,12 @@
 //   amplitudes), unless both qubits are register slots;
 // - CX and SWAP gates change no amplitudes: they change the labels (tile
 //   indices) a thread's amplitudes carry, and the next re-mapping writes them
-//   to their new places.
+//   to their new places;
+// - an X moves on through the gates after it into the next one-qubit unitary
+//   on its qubit, at no cost, or is a label change where there is none.  A
+//   unitary whose rotation is by more than 45 degrees is an X after one by
+//   less, so tangents are small, and an X, a Y or any other unitary without a
+//   diagonal moves the amplitudes and nothing else.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -69,6 +74,7 @@ PlanOptions factored_plan_options(int dtype, int n) {
     PlanOptions o = default_plan_options(dtype, n);
     o.f_tile_bits = std::min(n, dtype == QK_C128 ? 10 : 12);
     o.f_reg_bits = std::min(o.f_tile_bits, dtype == QK_C128 ? 4 : 5);
+    o.f_flips = 1;
     return o;
 }
 
@@ -80,6 +86,7 @@ PlanOptions factored_adjoint_options(int dtype, int n) {
     if (dtype == QK_C128) {
         o.f_tile_bits = std::min(n, 9);
         o.f_reg_bits = std::min(o.f_tile_bits, 3);
+        o.f_flips = 1;
     }
     return o;
 }
@@ -189,65 +196,43 @@ void merge_runs(std::vector<Op> &ops, int n) {
 cl scalar_of(const Op &op) {
     return {(long double)op.m[6] + op.m[8], (long double)op.m[7] + op.m[9]};
 }
+void set_scalar(Op &op, cl g) {
+    cset(op.m, 3, to_double(g));
+    op.m[8] = (double)(g.real() - op.m[6]);
+    op.m[9] = (double)(g.imag() - op.m[7]);
+}
 
-// OP_DENSE1 with phases aux -> OP_K.  t is the tangent of the rotation, as
-// large as it is: x - t y and t x + y round like the rotation's own rows.
-// Only a rotation by (nearly) pi has no usable tangent; its t is capped where
-// the other column's share, 1 / t, is far below a rounding.  t and the phases
-// are rounded to the state's type here and the scalar's magnitude taken from
-// the rounded values, so that their rounding does not change the norm.
+// OP_DENSE1 with phases aux and no tangent above 16 -> OP_K and its scalar.  t and the phases are rounded to the state's type here
+// and the scalar's magnitude taken from the rounded values, so that their
+// rounding does not change the norm.
 // ph: a phase the upper half still lacks; *defer: not null where the left
 // phase moves on instead, to be returned there.
-void extract(Op &op, int dtype, cl ph, cl *defer) {
-    constexpr long double cap = 0x1p64L;
+cl extract(Op &op, int dtype, cl ph, cl *defer) {
     auto rounded = [&](long double x) { return dtype == QK_C64 ? (double)(float)x : (double)x; };
     const cl a = cget(op.m, 0), b = cl(cget(op.m, 1)) * ph, c = cget(op.m, 2), d = cl(cget(op.m, 3)) * ph;
     const bool right = op.aux & kRightPhase, left = op.aux & kLeftPhase;
-    // M = g [[1, -t l], [p t, p l]]; from the column entry c = g p t where
-    // the tangent is large, from a = g where it is not
-    const bool large = !(std::norm(a) >= std::norm(c));
-    // the phases keep what modulus the entries give them: a matrix that is a
-    // unitary to rounding is met to rounding in all its entries
-    cl l = 1, p = 1, u = a;   // u: a multiple of g
+    // M = g [[1, -t l], [p t, p l]].  The phases keep what modulus the
+    // entries give them: a matrix that is a unitary to rounding is met to
+    // rounding in all its entries
+    const cl q = c / a;
+    cl l = 1, p = 1;
     long double tan;
-    if (!large) {
-        const cl q = c / a;
-        if (!left) {
-            tan = q.real();
-            if (right) l = d / a;
-        } else if (!right) {
-            tan = -(b / a).real();
-            p = d / a;
-        } else {
-            tan = std::sqrt(std::abs(q * b) / std::abs(d));
-            if (tan > 0) p = q / tan;
-            l = d / a / p;
-        }
+    if (!left) {
+        tan = q.real();
+        if (right) l = d / a;
+    } else if (!right) {
+        tan = -(b / a).real();
+        p = d / a;
     } else {
-        long double k;   // 1 / tan
-        u = c;
-        if (!left) {
-            k = (a / c).real();
-            if (right) l = -b / c;
-        } else if (!right) {
-            k = -(a / b).real();
-            p = -c / b;
-            u = c / p;
-        } else {
-            const long double ra = std::abs(a);
-            u = ra > 0 ? a / ra : cl(1);
-            k = std::sqrt(ra * std::abs(d) / (std::abs(b) * std::abs(c)));
-            p = unit(c / u);
-            l = -b / u / std::abs(c);
-        }
-        if (std::signbit(k)) u = -u;   // (k may be -0)
-        tan = std::fabs(k) * cap < 1 ? std::copysign(cap, k) : 1 / k;
+        tan = std::sqrt(std::abs(q * b) / std::abs(d));
+        if (tan > 0) p = q / tan;
+        l = d / a / p;
     }
     const double t = rounded(tan);
     const cd lr(rounded(l.real()), rounded(l.imag()));
     cd pr(rounded(p.real()), rounded(p.imag()));
     const long double nl = std::norm(cl(lr)), np = defer ? std::norm(p) : std::norm(cl(pr)), tt = (long double)t * t;
-    const cl g = unit(u) * std::sqrt((std::norm(a) + std::norm(b) + std::norm(c) + std::norm(d)) /
+    const cl g = unit(a) * std::sqrt((std::norm(a) + std::norm(b) + std::norm(c) + std::norm(d)) /
                                      (1 + tt * nl + np * (tt + nl)));
     if (defer) *defer = p, pr = 1;
     op.kind = OP_K;
@@ -255,9 +240,7 @@ void extract(Op &op, int dtype, cl ph, cl *defer) {
     op.m[0] = t;
     cset(op.m, 1, lr);
     cset(op.m, 2, pr);
-    cset(op.m, 3, to_double(g));
-    op.m[8] = (double)(g.real() - op.m[6]);
-    op.m[9] = (double)(g.imag() - op.m[7]);
+    return g;
 }
 
 bool is_sign(cd f) { return f.real() == -1.0 && std::fabs(f.imag()) < 2e-16; }   // CP(pi)
@@ -270,25 +253,57 @@ bool diagonal_on(const Op &op, int q) {
     }
 }
 
-// Merged ops -> OP_K, OP_PHASE1, OP_PHASE2, OP_CX, OP_SWAP2, OP_GRAD, OP_PERM
-// and a scalar of the whole list.  `scaled`: the list has ops with a scalar.
-void factor(std::vector<Op> &ops, int n, int dtype, cl &scale, bool &scaled) {
+// An X on q after op: OP_X, or two rotations by 45 degrees (the sums of an
+// amplitude with zero are exact).
+void push_x(std::vector<Op> &out, int q, const PlanOptions &o) {
+    Op x;
+    std::memset(&x, 0, sizeof x);
+    x.nq = 1;
+    x.q[0] = q;
+    x.kind = o.f_flips ? OP_X : OP_K;
+    if (!o.f_flips) {
+        x.aux = kRightPhase;
+        x.m[0] = 1;
+        cset(x.m, 1, -1);
+        cset(x.m, 2, 1);
+        set_scalar(x, std::sqrt(0.5L));
+        out.push_back(x);
+        cset(x.m, 1, 1);
+    }
+    out.push_back(x);
+}
+
+// Merged ops -> OP_K, OP_PHASE1, OP_PHASE2, OP_CX, OP_SWAP2, OP_GRAD, OP_PERM,
+// OP_X and a scalar the list lacks at its end.  `scaled`: it has ops with a
+// scalar.
+void factor(std::vector<Op> &ops, int n, const PlanOptions &o, cl &tail, bool &scaled) {
     // next[i] bit k: after op i, the next op on q[k] that is not diagonal
-    // there is a one-qubit unitary, which takes in a phase on that qubit
-    std::vector<char> dense(n, 0), next(ops.size(), 0);
+    // there is a one-qubit unitary, which takes in a phase on that qubit;
+    // bit 2 + k: some one-qubit unitary follows there, which takes in an X;
+    // bit 4 + k: and so on all qubits that CX gates carry the X to on the way
+    std::vector<char> dense(n, 0), later(n, 0), taken(n, 0), next(ops.size(), 0);
+    auto moved = [](std::vector<char> &f, const Op &op) {   // what follows an op's qubits through its swaps
+        const int k = op.kind == OP_SWAP2 || op.kind == OP_PERM ? op.nq / 2 : 0;
+        for (int i = 0; i < k; ++i) std::swap(f[op.q[i]], f[op.q[k + i]]);
+    };
     for (size_t i = ops.size(); i-- > 0;) {
         const Op &op = ops[i];
-        for (int k = 0; k < std::min<int>(op.nq, 2); ++k) next[i] |= dense[op.q[k]] ? 1 << k : 0;
+        for (int k = 0; k < std::min<int>(op.nq, 2); ++k)
+            next[i] |= (dense[op.q[k]] ? 1 << k : 0) | (later[op.q[k]] ? 4 << k : 0) | (taken[op.q[k]] ? 16 << k : 0);
         if (op.kind == OP_PERM) std::fill(dense.begin(), dense.end(), 0);
         else
             for (int k = 0; k < op.nq; ++k)
                 if (!diagonal_on(op, op.q[k])) dense[op.q[k]] = op.kind == OP_DENSE1;
+        moved(later, op);
+        moved(taken, op);
+        if (op.kind == OP_DENSE1) later[op.q[0]] = taken[op.q[0]] = 1;
+        if (op.kind == OP_CX) taken[op.q[op.aux]] &= taken[op.q[1 - op.aux]];
     }
     std::vector<cl> ph(n, 1);
-    std::vector<char> has(n, 0);
+    std::vector<char> has(n, 0), flip(n, 0);   // flip: an X on its way
     std::vector<Op> out;
     out.reserve(ops.size());
-    scale = 1;
+    tail = 1;   // scalar of the ops so far that no OP_K has taken
     scaled = false;
     auto phase1 = [&](int q, cl p, bool deferred) {
         if (deferred) {
@@ -296,41 +311,72 @@ void factor(std::vector<Op> &ops, int n, int dtype, cl &scale, bool &scaled) {
             has[q] = 1;
             return;
         }
-        Op o;
-        std::memset(&o, 0, sizeof o);
-        o.kind = OP_PHASE1;
-        o.nq = 1;
-        o.q[0] = q;
-        cset(o.m, 0, to_double(p));
-        out.push_back(o);
+        Op x;
+        std::memset(&x, 0, sizeof x);
+        x.kind = OP_PHASE1;
+        x.nq = 1;
+        x.q[0] = q;
+        cset(x.m, 0, to_double(p));
+        out.push_back(x);
     };
     for (size_t i = 0; i < ops.size(); ++i) {
         Op op = ops[i];
         const int q = op.q[0];
+        const bool f0 = flip[q], f1 = op.nq > 1 && flip[op.q[1]];
+        auto swapped = [&](int j, int k) {   // entries j and k of its matrix
+            const cd x = cget(op.m, j);
+            cset(op.m, j, cget(op.m, k));
+            cset(op.m, k, x);
+        };
         switch (op.kind) {
-        case OP_DENSE1:
+        case OP_DENSE1: {
             scaled = true;
-            {
-                const cl f = has[q] ? ph[q] : cl(1);
-                if (has[q]) op.aux |= kRightPhase;
+            const cl rest = has[q] ? ph[q] : cl(1);
+            if (has[q]) op.aux |= kRightPhase;
+            has[q] = 0;
+            ph[q] = 1;
+            if (f0) swapped(0, 1), swapped(2, 3);
+            // An X that costs label changes (and with them re-mappings: 106
+            // against 97 ms on the 26-qubit HEA gradient, in segments of one
+            // and a half layers) is made of tangents above 16 alone.
+            flip[q] = std::norm(cget(op.m, 2)) > (next[i] & 16 ? 1 : 256) * std::norm(cget(op.m, 0));
+            if (flip[q]) swapped(0, 2), swapped(1, 3);
+            // (a rotation beside an X is one with a factor -1 on the right)
+            if (f0 || flip[q]) op.aux |= kRightPhase;
+            const cl a = cget(op.m, 0);
+            if (cget(op.m, 1) == 0.0 && cget(op.m, 2) == 0.0 && std::fabs(std::norm(a) - 1) < 1e-15L) {
+                tail *= a;   // a diagonal is left; unit entries: no gradient sees where its scalar goes
+                const cl p = cl(cget(op.m, 3)) / a * rest;
+                if (p != cl(1)) phase1(q, p, next[i] & 1);
+            } else {
                 const bool defer = (op.aux & kLeftPhase) && (next[i] & 1);
-                extract(op, dtype, f, defer ? &ph[q] : nullptr);
+                set_scalar(op, tail * extract(op, o.dtype, rest, defer ? &ph[q] : nullptr));
+                tail = 1;
                 has[q] = defer;
                 if (defer) op.aux &= ~kLeftPhase;
-                else ph[q] = 1;
+                out.push_back(op);
             }
-            out.push_back(op);
+            if (flip[q] && !(next[i] & 4)) push_x(out, q, o), flip[q] = 0;
             break;
-        case OP_PHASE1: phase1(q, cget(op.m, 0), next[i] & 1); break;
+        }
+        case OP_PHASE1: {
+            const cl p = cget(op.m, 0);
+            if (f0) tail *= p, scaled = true;
+            phase1(q, f0 ? cl(1) / p : p, next[i] & 1);
+            break;
+        }
         case OP_DIAG1:
+            if (f0) swapped(0, 1);
             scaled = true;
-            scale *= cl(cget(op.m, 0));
+            tail *= cl(cget(op.m, 0));
             phase1(q, cl(cget(op.m, 1)) / cl(cget(op.m, 0)), next[i] & 1);
             break;
         case OP_DIAG2: {
+            if (f0) swapped(0, 1), swapped(2, 3);
+            if (f1) swapped(0, 2), swapped(1, 3);
             const cl d0 = cget(op.m, 0), d1 = cget(op.m, 1), d2 = cget(op.m, 2), d3 = cget(op.m, 3);
             scaled = true;
-            scale *= d0;
+            tail *= d0;
             phase1(op.q[0], d1 / d0, next[i] & 1);
             phase1(op.q[1], d2 / d0, next[i] & 2);
             op.kind = OP_PHASE2;
@@ -338,7 +384,15 @@ void factor(std::vector<Op> &ops, int n, int dtype, cl &scale, bool &scaled) {
             out.push_back(op);
             break;
         }
-        case OP_PHASE2:
+        case OP_PHASE2: {
+            if (f0 || f1) {   // w^(b0 b1) with b = 1 - b' on the flipped qubits
+                const cl w = cget(op.m, 0);
+                scaled = true;
+                if (f0 && f1) tail *= w;
+                if (f1) phase1(op.q[0], f0 ? cl(1) / w : w, next[i] & 1);
+                if (f0) phase1(op.q[1], f1 ? cl(1) / w : w, next[i] & 2);
+                if (f0 != f1) cset(op.m, 0, to_double(cl(1) / w));
+            }
             // CP(pi) is (-1, 1.2e-16) and runs as a change of sign.  What is
             // dropped, exp(i e b0 b1), goes where it costs nothing: b0 b1 is
             // (b0 + b1) / 2 - 1 / 4, b0 / 2 or 1 / 4 on average (left out, it
@@ -348,13 +402,47 @@ void factor(std::vector<Op> &ops, int n, int dtype, cl &scale, bool &scaled) {
                 const int k0 = (next[i] & 1) != 0, k1 = (next[i] & 2) != 0;
                 if (k0) phase1(op.q[0], std::polar(1.0L, e / 2), true);
                 if (k1) phase1(op.q[1], std::polar(1.0L, e / 2), true);
-                scale *= std::polar(1.0L, e * (1 - k0 - k1) / 4);
+                tail *= std::polar(1.0L, e * (1 - k0 - k1) / 4);
                 scaled = true;
             }
             out.push_back(op);
             break;
-        default: out.push_back(op); break;
         }
+        case OP_CX: {
+            out.push_back(op);
+            const int ctl = op.q[op.aux], tgt = op.q[1 - op.aux];
+            flip[tgt] ^= flip[ctl];
+            if (flip[tgt] && !(next[i] & (4 << (1 - op.aux)))) push_x(out, tgt, o), flip[tgt] = 0;
+            break;
+        }
+        case OP_GRAD:
+            if (f0) {   // X G X: the Y and Z parts change sign
+                const int gen = (int)op.m[0];
+                if (gen == 2 || gen == 3) {
+                    op.m[0] = 4;
+                    op.m[gen + 1] = 1;
+                }
+                for (int k : {3, 4, 6, 7}) op.m[k] = -op.m[k];
+            }
+            out.push_back(op);
+            break;
+        default:
+            moved(flip, op);
+            out.push_back(op);
+            break;
+        }
+    }
+    if (tail != cl(1) && std::all_of(out.begin(), out.end(), [](const Op &x) { return x.kind == OP_PERM; })) {
+        // the scalar is all there is to do: on a unitary of its own
+        Op x;
+        std::memset(&x, 0, sizeof x);
+        x.kind = OP_K;
+        x.nq = 1;
+        cset(x.m, 1, 1);
+        cset(x.m, 2, 1);
+        set_scalar(x, tail);
+        tail = 1;
+        out.insert(out.begin(), x);
     }
     ops.swap(out);
 }
@@ -366,7 +454,7 @@ bool is_work(const Op &op) { return op.kind == OP_K || op.kind == OP_GRAD; }
 // Tile bits an op needs (its register slot, or the labels it changes).
 int tile_bits_of(const Op &op, int (&b)[2]) {
     switch (op.kind) {
-    case OP_K: case OP_GRAD: b[0] = op.q[0]; return 1;
+    case OP_K: case OP_GRAD: case OP_X: b[0] = op.q[0]; return 1;
     case OP_CX: b[0] = op.q[1 - op.aux]; return 1;
     case OP_SWAP2: b[0] = op.q[0]; b[1] = op.q[1]; return 2;
     default: return 0;
@@ -379,8 +467,9 @@ struct Builder {
     HostPlan &plan;
     const PlanOptions &opts;
     bool lookahead;
-    cl carry;            // scalar the stored state still lacks
+    cl tail;             // scalar the ops leave out
     bool scaled;
+    cl carry = 1;        // scalar of the ops so far, which the stored state lacks
     int grad_base = 0;
     bool mapped = false;   // the last step is a re-mapping
     // the TOP_LAYER being collected: its unitaries by slot
@@ -434,7 +523,7 @@ struct Builder {
             x.nb = (uint8_t)tile_bits_of(op, b);
             for (int k = 0; k < op.nq; ++k) x.q[k] = (uint8_t)op.q[k], x.diag[k] = diagonal_on(op, op.q[k]);
             for (int k = 0; k < x.nb; ++k) x.b[k] = (uint8_t)b[k];
-            x.work = is_work(op) ? 4 : op.kind == OP_CX || op.kind == OP_SWAP2 ? 1 : 0;
+            x.work = is_work(op) ? 4 : x.nb ? 1 : 0;
         }
     }
 
@@ -582,7 +671,8 @@ struct Builder {
         std::vector<char> keep(take.size(), 0), need(n, 0);   // need: by kept ops, as touched
         for (size_t k = take.size(); k-- > 0;) {
             const Op &op = ops[take[k]];
-            bool kp = is_work(op), later = false;
+            // (an X comes after the qubit's last unitary)
+            bool kp = is_work(op) || op.kind == OP_X, later = false;
             for (int j = 0; j < op.nq; ++j) {
                 const bool dg = diagonal_on(op, op.q[j]);
                 kp = kp || need[op.q[j]] > (dg ? 1 : 0);
@@ -676,7 +766,7 @@ struct Builder {
         return cnt;
     }
 
-    // CX and SWAP labels (and, once no work is left, the remaining phases).
+    // CX, SWAP and X labels (and, once no work is left, the remaining phases).
     bool run_labels(Pass &P) {
         bool changed = false;
         std::vector<int> ph;
@@ -700,7 +790,10 @@ struct Builder {
                         --P.left;
                     }
                     changed = true;
-                    if (op.kind == OP_CX) {
+                    if (op.kind == OP_X) {
+                        label(P, op.q[0], -1);
+                        P.dirty[op.q[0]] = 2;
+                    } else if (op.kind == OP_CX) {
                         label(P, op.q[1 - op.aux], op.q[op.aux]);
                         P.dirty[op.q[op.aux]] = std::max<char>(P.dirty[op.q[op.aux]], 1);
                         P.dirty[op.q[1 - op.aux]] = 2;
@@ -772,10 +865,10 @@ struct Builder {
     uint8_t code(const Pass &P, int q) const {
         return P.local[q] >= 0 ? (uint8_t)P.local[q] : (uint8_t)(kOuterFlag | q);
     }
-    void label(const Pass &P, int target, int control) {
+    void label(const Pass &P, int target, int control) {   // (control -1: an X)
         TOp &t = step(TOP_LCX);
         t.a = (uint8_t)P.local[target];
-        t.b = code(P, control);
+        t.b = control < 0 ? kNoQubit : code(P, control);
     }
     void remap(Pass &P, const std::vector<int> &Q, bool dirty) {
         P.Q = Q;
@@ -824,14 +917,19 @@ struct Builder {
             const cd f = cget(o.m, 0);
             cond.push_back({x < 0 ? kNoQubit : (uint8_t)(code(P, x) | (is_sign(f) ? kSignFlag : 0)), f});
         }
-        // amplitudes grow by 1 / |scalar|; before their magnitude leaves a
-        // quarter of the type's exponent range it is set back
-        const double range = plan.dtype == QK_C128 ? 0x1p-200 : 0x1p-60;
-        if (std::abs(carry * scalar_of(op)) < range) {
-            const double f = rounded((double)std::abs(carry));
-            step(TOP_SCALE);
-            push(f);
-            carry /= f;
+        // Amplitudes grow by 1 / |scalar|.  Before their magnitude is 2^16
+        // (2^32 for complex128) times their own it is set back, by a power of
+        // two: exact, and so much closer to the type's largest number an
+        // amplitude may be.
+        const long double range = plan.dtype == QK_C128 ? 0x1p-32L : 0x1p-16L, after = std::abs(carry * scalar_of(op));
+        if (!(after >= range && after <= 1 / range)) {
+            const int lim = plan.dtype == QK_C128 ? 500 : 60;
+            const double f = std::ldexp(1.0, std::max(-lim, std::min(lim, std::ilogb(std::abs(carry)))));
+            if (f != 1) {
+                step(TOP_SCALE);
+                push(f);
+                carry /= f;
+            }
         }
         carry *= scalar_of(op);
         bool simple = true;   // conditions that only change the sign
@@ -888,7 +986,6 @@ struct Builder {
             push(cget(op.m, 2));
         }
     }
-    double rounded(double x) const { return plan.dtype == QK_C64 ? (double)(float)x : x; }
     void emit_grad(Pass &P, const Op &op) {
         // both states lack the factor carry: the sums grow by its square
         const double f = (double)std::norm(carry);
@@ -1017,7 +1114,7 @@ struct Builder {
         if (scaled && last_pass) {
             TOp &t = step(TOP_SCALE);
             t.b = 1;
-            push({(double)carry.real(), (double)carry.imag()});
+            push(to_double(carry * tail));
             carry = 1;
         }
         d.nprog = (int)plan.ops.size() - d.prog0;
@@ -1042,7 +1139,7 @@ struct Builder {
 // The candidates of a plan: op lists, each in both orders and with both ways
 // to choose tiles.  All are cut into passes; of those with the fewest passes
 // the first and the last are compiled, the one with fewer re-mappings kept.
-int build_best(const std::vector<std::vector<Op>> &lists, const std::vector<cl> &scale, const std::vector<char> &scaled,
+int build_best(const std::vector<std::vector<Op>> &lists, const std::vector<cl> &tail, const std::vector<char> &scaled,
                int n, const PlanOptions &o, int nstates, HostPlan &plan) {
     PlanOptions fo = o;
     fo.tile_bits = o.f_tile_bits;
@@ -1066,7 +1163,7 @@ int build_best(const std::vector<std::vector<Op>> &lists, const std::vector<cl> 
         c.ops = lists[list];
         if (variant % 2) asap_order(c.ops, n);
         HostPlan hp = empty;
-        Builder b{c.ops, n, o.f_tile_bits, o.f_reg_bits, L, hp, o, variant >= 2, scale[list], scaled[list] != 0};
+        Builder b{c.ops, n, o.f_tile_bits, o.f_reg_bits, L, hp, o, variant >= 2, tail[list], scaled[list] != 0};
         const int rc = b.partition();
         c.parts.swap(b.parts);
         return rc;
@@ -1091,7 +1188,7 @@ int build_best(const std::vector<std::vector<Op>> &lists, const std::vector<cl> 
     for (Candidate *c : {&first, &last}) {
         if (c == &last && !two) break;
         HostPlan hp = empty;
-        Builder b{c->ops, n, o.f_tile_bits, o.f_reg_bits, L, hp, o, false, scale[c->list], scaled[c->list] != 0};
+        Builder b{c->ops, n, o.f_tile_bits, o.f_reg_bits, L, hp, o, false, tail[c->list], scaled[c->list] != 0};
         b.make_lite();
         b.parts.swap(c->parts);
         int rc = b.compile_parts();
@@ -1126,7 +1223,7 @@ static int forward(const qk_gate *gates, size_t ng, int n, const PlanOptions &o,
     }
     // SWAP gates as label steps, or as renamings too
     std::vector<std::vector<Op>> lists;
-    std::vector<cl> scale;
+    std::vector<cl> tail;
     std::vector<char> scaled;
     for (int rename = 0; rename <= (swaps ? 1 : 0); ++rename) {
         std::vector<Op> ops = lowered;
@@ -1134,12 +1231,12 @@ static int forward(const qk_gate *gates, size_t ng, int n, const PlanOptions &o,
         merge_runs(ops, n);
         cl f;
         bool has;
-        factor(ops, n, o.dtype, f, has);
+        factor(ops, n, o, f, has);
         lists.push_back(std::move(ops));
-        scale.push_back(f);
+        tail.push_back(f);
         scaled.push_back(has);
     }
-    return build_best(lists, scale, scaled, n, o, 1, plan);
+    return build_best(lists, tail, scaled, n, o, 1, plan);
 }
 
 static int adjoint(const qk_gate *gates, size_t ng, const int32_t *pidx, int n, const PlanOptions &o, HostPlan &plan) {
@@ -1169,10 +1266,10 @@ static int adjoint(const qk_gate *gates, size_t ng, const int32_t *pidx, int n, 
     hoist_gradients(ops, n);
     merge_runs(ops, n);
     pair_gradients(ops);
-    cl scale;
+    cl tail;
     bool scaled;
-    factor(ops, n, o.dtype, scale, scaled);
-    return build_best({ops}, {scale}, {scaled}, n, o, 2, plan);
+    factor(ops, n, o, tail, scaled);
+    return build_best({ops}, {tail}, {scaled}, n, o, 2, plan);
 }
 
 int plan_forward(const qk_gate *gates, size_t ng, int n, const PlanOptions &o, HostPlan &plan) {

@@ -253,7 +253,7 @@ __device__ __forceinline__ void run_steps(C (&v)[R], C (&w)[NS == 2 ? R : 1], un
                 for (int s = 0; s < LOG2R; ++s) bm[s] = 1u << ((s < 4 ? slots >> (8 * (s & 3)) : slot5) & 31);
             }
             if (b & kOuterFlag) {
-                tb ^= ((uint32_t)(base >> (b & 0x3F)) & 1u) << a;
+                tb ^= (uint32_t)code_bit(b, base, tb) << a;
             } else {
                 tb ^= ((tb >> b) & 1u) << a;
 #pragma unroll

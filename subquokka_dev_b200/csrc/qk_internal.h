@@ -31,6 +31,7 @@ enum OpKind : int32_t {
     OP_K = 11,  // factored one-qubit unitary on q[0], without its scalar (planner-made, qk_factor.cpp):
                 // right phase m[2..3] on the upper half, then x' = x - t y, y' = t x + y, t = m[0], then
                 // left phase m[4..5]; scalar m[6..7]; aux = kRightPhase | kLeftPhase
+    OP_X = 12,  // flip bit q[0] (planner-made, qk_factor.cpp)
 };
 constexpr int kRightPhase = 1, kLeftPhase = 2;
 
@@ -125,7 +126,8 @@ enum TOpKind : uint8_t {
     // kLayerWords, a sign, the parity of (tile label & w[s]) and (tile number & u[s]); the next two
     // words hold u, five 32-bit values, and w, five 16-bit values.  Then x' = x - t y, y' = t x + y
     TOP_LAYER = 14,
-    TOP_LCX = 15,   // label step: tile bit a ^= qubit code b (a CX whose swap the next TOP_REMAP performs)
+    TOP_LCX = 15,   // label step: tile bit a ^= qubit code b (a CX whose swap the next TOP_REMAP performs),
+                    // b = kNoQubit: flipped (an X; programs with f_flips)
     TOP_PH2 = 16,   // 16 + slot_pair(a, b): amplitude *= coef[0] where slots a and b are 1
     TOP_LAM = 28,   // pending factor of the next TOP_LAYER *= the entries of two tables: coef[i], i the
                     // bits of the first four condition codes in bits, and (nbits > 4)
@@ -216,6 +218,7 @@ struct PlanOptions {
     // plan_forward / plan_adjoint: tile and register bits of factored programs,
     // which are made where they can be (0: general programs only)
     int f_tile_bits = 0, f_reg_bits = 0;
+    int f_flips = 0;      // 1: factored programs may flip a tile bit (TOP_LCX with kNoQubit); 0: two rotations instead
     int threads = 0;      // 1: the factored planner tries its candidates on several host threads
 };
 
