@@ -202,7 +202,7 @@ void set_scalar(Op &op, cl g) {
     op.m[9] = (double)(g.imag() - op.m[7]);
 }
 
-// OP_DENSE1 with phases aux and no tangent above 16 -> OP_K and its scalar.  t and the phases are rounded to the state's type here
+// OP_DENSE1 with phases aux and no tangent above 2^10 -> OP_K and its scalar.  t and the phases are rounded to the state's type here
 // and the scalar's magnitude taken from the rounded values, so that their
 // rounding does not change the norm.
 // ph: a phase the upper half still lacks; *defer: not null where the left
@@ -338,8 +338,8 @@ void factor(std::vector<Op> &ops, int n, const PlanOptions &o, cl &tail, bool &s
             if (f0) swapped(0, 1), swapped(2, 3);
             // An X that costs label changes (and with them re-mappings: 106
             // against 97 ms on the 26-qubit HEA gradient, in segments of one
-            // and a half layers) is made of tangents above 16 alone.
-            flip[q] = std::norm(cget(op.m, 2)) > (next[i] & 16 ? 1 : 256) * std::norm(cget(op.m, 0));
+            // and a half layers) is made of tangents above 2^10 alone.
+            flip[q] = std::norm(cget(op.m, 2)) > (next[i] & 16 ? 1 : 0x1p20) * std::norm(cget(op.m, 0));
             if (flip[q]) swapped(0, 2), swapped(1, 3);
             // (a rotation beside an X is one with a factor -1 on the right)
             if (f0 || flip[q]) op.aux |= kRightPhase;
@@ -523,7 +523,7 @@ struct Builder {
             x.nb = (uint8_t)tile_bits_of(op, b);
             for (int k = 0; k < op.nq; ++k) x.q[k] = (uint8_t)op.q[k], x.diag[k] = diagonal_on(op, op.q[k]);
             for (int k = 0; k < x.nb; ++k) x.b[k] = (uint8_t)b[k];
-            x.work = is_work(op) ? 4 : x.nb ? 1 : 0;
+            x.work = is_work(op) ? 4 : op.kind == OP_CX || op.kind == OP_SWAP2 ? 1 : 0;
         }
     }
 

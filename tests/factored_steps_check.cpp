@@ -14,7 +14,7 @@
 //   rms in the 2-norm at most, independent: 3.3e-7, three times that), in
 //   float arithmetic within 90 x 4 x 2^-24 = 2.2e-5;
 // - states of amplitude 1e30 (complex64) and 1e290: finite and as accurate;
-// - every tangent at most 16, every real scale a power of two other than 1;
+// - every tangent at most 2^10, every real scale a power of two other than 1;
 // - adjoint plans against the direct backward sweep, within 1e-12, gradients
 //   of circuits with H (whose constant is 1.1e-11 off a unitary's) 1e-9.
 #include "dense_sim.h"
@@ -197,7 +197,7 @@ template <typename T> struct Emulator {
     }
     void pair(const TOp &op, Z<T> first, Z<T> second, bool neg, Z<T> pend, Z<T> &x, Z<T> &y) {
         const T t = first.real();
-        if (!(std::fabs(t) <= 16 * (1 + 1e-6))) die("a tangent above 16");
+        if (!(std::fabs(t) <= 1024 * (1 + 1e-6))) die("a tangent above 2^10");
         Z<T> l = (op.b & qk::kLayerPending) ? pend : second;
         if (neg) l = -l;
         const Z<T> z = times(l, y), x0 = x;
