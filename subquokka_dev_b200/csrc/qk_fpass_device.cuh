@@ -75,19 +75,51 @@ __device__ __forceinline__ void k_unitary(C (&v)[R], const C l, const T t) {
     }
 }
 
-// Value of a condition code that is the same for all of the thread's
-// amplitudes.
-__device__ __forceinline__ bool code_bit(uint32_t code, uint64_t base, uint32_t tb) {
-    if (code == kNoQubit) return true;
-    return (code & kOuterFlag) ? (base >> (code & 0x3F)) & 1 : (tb >> (code & 0x3F)) & 1;
-}
-
 // The sign bit of x flipped where s is odd.
 __device__ __forceinline__ double flip_sign(double x, uint32_t s) {
     return __hiloint2double(__double2hiint(x) ^ (int)(s << 31), __double2loint(x));
 }
 __device__ __forceinline__ float flip_sign(float x, uint32_t s) {
     return __uint_as_float(__float_as_uint(x) ^ (s << 31));
+}
+
+// c + f a.
+template <typename C> __device__ __forceinline__ C madd(const C f, const C a, const C c) {
+    C r;
+    r.x = fma(f.x, a.x, fma(-f.y, a.y, c.x));
+    r.y = fma(f.x, a.y, fma(f.y, a.x, c.y));
+    return r;
+}
+// A full unitary on slot S, without its left phase: x' = x + B y, y' = F x + y.  As many multiply-adds as k_unitary,
+// but neither result can be written in place.
+template <int S, typename C, int R>
+__device__ __forceinline__ void k_full(C (&v)[R], const C B, const C F) {
+    if constexpr ((1 << S) < R) {
+#pragma unroll
+        for (int k = 0; k < R; ++k)
+            if (!(k & (1 << S))) {
+                const C x = v[k];
+                v[k] = madd(B, v[k | (1 << S)], x);
+                v[k | (1 << S)] = madd(F, x, v[k | (1 << S)]);
+            }
+    }
+}
+template <int S, typename C, int R> __device__ __forceinline__ void k_negate(C (&v)[R]) {
+    if constexpr ((1 << S) < R) {
+#pragma unroll
+        for (int k = 0; k < R; ++k)
+            if (k & (1 << S)) {
+                v[k].x = flip_sign(v[k].x, 1);
+                v[k].y = flip_sign(v[k].y, 1);
+            }
+    }
+}
+
+// Value of a condition code that is the same for all of the thread's
+// amplitudes.
+__device__ __forceinline__ bool code_bit(uint32_t code, uint64_t base, uint32_t tb) {
+    if (code == kNoQubit) return true;
+    return (code & kOuterFlag) ? (base >> (code & 0x3F)) & 1 : (tb >> (code & 0x3F)) & 1;
 }
 
 // Byte offset of register element kk under slot offsets sb.
@@ -199,6 +231,23 @@ __device__ __forceinline__ void run_steps(C (&v)[R], C (&w)[NS == 2 ? R : 1], un
                 QK_SG(0, 4) QK_SG(1, 4) QK_SG(2, 4) QK_SG(3, 4)
 #undef QK_SG
             }
+            if constexpr (sizeof(C) == sizeof(double2))   // (complex64 programs have none)
+                if (b & kLayerFull) {
+#define QK_F(S)                                                     \
+    if constexpr ((1 << S) < R)                                     \
+        if ((a >> S) & 1) {                                         \
+            if ((neg >> S) & 1) {                                   \
+                k_negate<S>(v);                                     \
+                if constexpr (NS == 2) k_negate<S>(w);              \
+            }                                                       \
+            k_full<S>(v, m[0], m[1]);                               \
+            if constexpr (NS == 2) k_full<S>(w, m[0], m[1]);        \
+            m += 2;                                                 \
+        }
+                    QK_F(0) QK_F(1) QK_F(2) QK_F(3) QK_F(4)
+#undef QK_F
+                    break;
+                }
             const bool pending = b & kLayerPending;
 #define QK_K(S)                                                     \
     if constexpr ((1 << S) < R)                                     \

@@ -30,10 +30,11 @@ enum OpKind : int32_t {
     OP_CDENSE1 = 10,  // 2x2 on q[0]: m[0..7] where bit q[1] is 0, m[8..15] where it is 1 (planner-made)
     OP_K = 11,  // factored one-qubit unitary on q[0], without its scalar (planner-made, qk_factor.cpp):
                 // right phase m[2..3] on the upper half, then x' = x - t y, y' = t x + y, t = m[0], then
-                // left phase m[4..5]; scalar m[6..7]; aux = kRightPhase | kLeftPhase
+                // left phase m[4..5]; scalar m[6..7]; aux = kRightPhase | kLeftPhase.  aux & kFull:
+                // x' = x + B y, y' = F x + y, B = m[0..1], F = m[2..3], then the left phase
     OP_X = 12,  // flip bit q[0] (planner-made, qk_factor.cpp)
 };
-constexpr int kRightPhase = 1, kLeftPhase = 2;
+constexpr int kRightPhase = 1, kLeftPhase = 2, kFull = 4, kGiven = 8;   // kGiven: a circuit's own matrix (U1)
 
 struct Op {
     int32_t kind;
@@ -124,7 +125,9 @@ enum TOpKind : uint8_t {
     // Then for each slot s in a, ascending, a unitary with coefficients t and right phase: the slot's
     // upper half y takes the right phase (kLayerPending: the pending factor instead) and, with
     // kLayerWords, a sign, the parity of (tile label & w[s]) and (tile number & u[s]); the next two
-    // words hold u, five 32-bit values, and w, five 16-bit values.  Then x' = x - t y, y' = t x + y
+    // words hold u, five 32-bit values, and w, five 16-bit values.  Then x' = x - t y, y' = t x + y.
+    // With kLayerFull (programs with f_full) the coefficients are complex, B and F: y takes the sign alone,
+    // then x' = x + B y, y' = F x + y
     TOP_LAYER = 14,
     TOP_LCX = 15,   // label step: tile bit a ^= qubit code b (a CX whose swap the next TOP_REMAP performs),
                     // b = kNoQubit: flipped (an X; programs with f_flips)
@@ -135,7 +138,7 @@ enum TOpKind : uint8_t {
                     // the tile number
     TOP_SCALE = 29, // amplitude *= coef[0] (b = 1: complex, 0: its real part)
 };
-constexpr uint8_t kLayerWords = 0x20, kLayerSigns = 0x40, kLayerPending = 0x80;   // TOP_LAYER, high half of b
+constexpr uint8_t kLayerFull = 0x10, kLayerWords = 0x20, kLayerSigns = 0x40, kLayerPending = 0x80;   // TOP_LAYER, high half of b
 constexpr uint8_t kSignFlag = 0x40;   // condition codes of factored steps: the factor is -1
 // index of the slot pair a < b among 0..9 (five slots)
 constexpr int slot_pair(int a, int b) { return b * (b - 1) / 2 + a; }
@@ -219,6 +222,7 @@ struct PlanOptions {
     // which are made where they can be (0: general programs only)
     int f_tile_bits = 0, f_reg_bits = 0;
     int f_flips = 0;      // 1: factored programs may flip a tile bit (TOP_LCX with kNoQubit); 0: two rotations instead
+    int f_full = 0;       // 1: factored programs may hold layers of full unitaries (kLayerFull); 0: rotations only
     int threads = 0;      // 1: the factored planner tries its candidates on several host threads
 };
 

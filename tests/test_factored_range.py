@@ -1,6 +1,6 @@
 """Factored fused passes: gates that only move amplitudes are exact, and the
 amplitudes may be as large as their type allows, but for the growth the plans
-keep below 2^16 (complex64) and 2^32 (complex128).
+keep below 2^16 (complex64) and 2^48 (complex128).
 
 CPU: tests/factored_steps_check.cpp runs the programs as the engine plans them
 in the arithmetic of the state's type.  GPU: plans, subcircuit files and
