@@ -105,7 +105,7 @@ void cset(double *m, int k, cd z) {
     m[2 * k] = z.real();
     m[2 * k + 1] = z.imag();
 }
-cl unit(cl z) { return z / std::abs(z); }
+cl unit(cl z) { return z / std::sqrt(std::norm(z)); }
 cd to_double(cl z) { return {(double)z.real(), (double)z.imag()}; }
 
 // ---- gate list -> factored op list ------------------------------------------
@@ -226,7 +226,9 @@ cl extract(Op &op, int dtype, cl ph, bool full, cl *defer) {
         // out, the angle of -b c / (a d), is 0 in a unitary but not in a
         // rounded one; shared among the entries as the least squares have it,
         // it is off in the 2-norm.
-        const long double sa = std::norm(a), sb = std::norm(b), e = std::arg(-b * c / (a * d)),
+        const cl bc = -b * c, ad = a * d, turn = bc * std::conj(ad);
+        const long double sa = std::norm(a), sb = std::norm(b),
+                          e = std::fabs(turn.imag()) < 1e-8L * turn.real() ? turn.imag() / turn.real() : std::arg(turn),
                           off = e * std::sqrt(sa * sb) / (sa + sb) / 2;
         if (full && std::fabs(off) > kFullAbove) {
             const cd B = to_double(b / a), F = to_double(c / d);
@@ -241,7 +243,8 @@ cl extract(Op &op, int dtype, cl ph, bool full, cl *defer) {
             cset(op.m, 2, defer ? cd(1) : to_double(p));
             return g;
         }
-        const cl up = std::polar(1.0L, e * sb / (sa + sb) / 2), down = std::polar(1.0L, -e * sa / (sa + sb) / 2);
+        auto turned = [](long double x) { return std::fabs(x) < 1e-8L ? cl(1 - x * x / 2, x) : std::polar(1.0L, x); };
+        const cl up = turned(e * sb / (sa + sb) / 2), down = turned(-e * sa / (sa + sb) / 2);
         a *= up, d *= up, b *= down, c *= down;
     }
     // M = g [[1, -t l], [p t, p l]].  The phases keep what modulus the
@@ -257,7 +260,7 @@ cl extract(Op &op, int dtype, cl ph, bool full, cl *defer) {
         tan = -(b / a).real();
         p = d / a;
     } else {
-        tan = std::sqrt(std::abs(q * b) / std::abs(d));
+        tan = std::sqrt(std::sqrt(std::norm(q * b) / std::norm(d)));
         if (tan > 0) p = q / tan;
         l = d / a / p;
     }
@@ -502,14 +505,63 @@ int tile_bits_of(const Op &op, int (&b)[2]) {
     }
 }
 
+// What the walks below look at, 16 bytes an op.
+struct Lite {
+    uint16_t cost;
+    uint8_t nq, nb, work, perm;
+    uint8_t q[2], diag[2], b[2];   // qubits, whether diagonal there, tile bits
+};
+
+// A factored op list in its two orders.
+struct List {
+    std::vector<Op> ops;
+    cl tail = 1;              // scalar the ops leave out
+    bool scaled = false;
+    std::vector<Lite> lite;
+    std::vector<size_t> order[2], rank[2];   // the ops as given and in ASAP layers; an op's place there
+};
+
+// Bytes of a pass's shared memory an op adds: steps, coefficients, accumulators.
+size_t cost(const Op &op, size_t c, int threads_log) {
+    switch (op.kind) {
+    case OP_K: return 40 + 3 * c;   // a share of the re-mappings included
+    case OP_GRAD: {
+        const size_t k = (int)op.m[0] == 5 ? 2 : 1;
+        return 16 + k * (2 * c + (sizeof(double) << threads_log));
+    }
+    case OP_SWAP2: return 64;
+    default: return 24 + 4 * c;   // (a condition's share of the tables)
+    }
+}
+void make_lite(List &list, size_t amp_bytes, int threads_log) {
+    const auto &ops = list.ops;
+    auto &lite = list.lite;
+    lite.resize(ops.size());
+    for (size_t i = 0; i < ops.size(); ++i) {
+        const Op &op = ops[i];
+        Lite &x = lite[i];
+        std::memset(&x, 0, sizeof x);
+        x.perm = op.kind == OP_PERM;
+        if (x.perm) continue;
+        x.cost = (uint16_t)std::min<size_t>(cost(op, amp_bytes, threads_log), 65535);
+        x.nq = (uint8_t)op.nq;
+        int b[2];
+        x.nb = (uint8_t)tile_bits_of(op, b);
+        for (int k = 0; k < op.nq; ++k) x.q[k] = (uint8_t)op.q[k], x.diag[k] = diagonal_on(op, op.q[k]);
+        for (int k = 0; k < x.nb; ++k) x.b[k] = (uint8_t)b[k];
+        x.work = is_work(op) ? 4 : op.kind == OP_CX || op.kind == OP_SWAP2 ? 1 : 0;
+    }
+}
+
 struct Builder {
-    const std::vector<Op> &ops;
+    const List &list;
+    bool asap;
     int n, T, r, L;
     HostPlan &plan;
     const PlanOptions &opts;
     bool lookahead;
-    cl tail;             // scalar the ops leave out
-    bool scaled;
+    const std::vector<Op> &ops = list.ops;
+    const std::vector<Lite> &lite = list.lite;
     cl carry = 1;        // scalar of the ops so far, which the stored state lacks
     int grad_base = 0;
     bool mapped = false;   // the last step is a re-mapping
@@ -530,54 +582,14 @@ struct Builder {
         const size_t tile = (amp_bytes() << T) * plan.nstates;
         return std::min<size_t>(48u << 10, (200u << 10) - tile);
     }
-    size_t cost(const Op &op) const {
-        const size_t c = amp_bytes();
-        switch (op.kind) {
-        case OP_K: return 40 + 3 * c;   // a share of the re-mappings included
-        case OP_GRAD: {
-            const size_t k = (int)op.m[0] == 5 ? 2 : 1;
-            return 16 + k * (2 * c + (sizeof(double) << (T - r)));
-        }
-        case OP_SWAP2: return 64;
-        default: return 24 + 4 * c;   // (a condition's share of the tables)
-        }
-    }
-
-    // What the walks below look at, 16 bytes an op.
-    struct Lite {
-        uint16_t cost;
-        uint8_t nq, nb, work, perm;
-        uint8_t q[2], diag[2], b[2];   // qubits, whether diagonal there, tile bits
-    };
-    std::vector<Lite> lite = {};
-    void make_lite() {
-        lite.resize(ops.size());
-        for (size_t i = 0; i < ops.size(); ++i) {
-            const Op &op = ops[i];
-            Lite &x = lite[i];
-            std::memset(&x, 0, sizeof x);
-            x.perm = op.kind == OP_PERM;
-            if (x.perm) continue;
-            x.cost = (uint16_t)std::min<size_t>(cost(op), 65535);
-            x.nq = (uint8_t)op.nq;
-            int b[2];
-            x.nb = (uint8_t)tile_bits_of(op, b);
-            for (int k = 0; k < op.nq; ++k) x.q[k] = (uint8_t)op.q[k], x.diag[k] = diagonal_on(op, op.q[k]);
-            for (int k = 0; k < x.nb; ++k) x.b[k] = (uint8_t)b[k];
-            x.work = is_work(op) ? 4 : op.kind == OP_CX || op.kind == OP_SWAP2 ? 1 : 0;
-        }
-    }
-
     // Walk pending ops in order; an op joins a pass on tile bits inB when no
     // op left out before it fails to commute with it on a shared qubit, its
     // tile bits are there (or, with grow, can be added) and the budget allows.
     // blocked: 1 an op diagonal on the qubit was left out, 2 another op.
     template <typename F>
-    size_t walk(const std::vector<size_t> &pending, std::vector<char> &inB, int *grow, F &&each) const {
+    void walk(const std::vector<size_t> &pending, std::vector<char> &inB, int *grow, F &&each) const {
         char blocked[64] = {0};
-        size_t used = 256, work = 0;
-        int open = 0;   // tile bits on which work can still join
-        for (int q = 0; q < n; ++q) open += inB[q];
+        size_t used = 256;
         const size_t lim = budget();
         for (size_t i : pending) {
             const Lite &op = lite[i];
@@ -593,19 +605,37 @@ struct Builder {
             }
             if (ok) {
                 used += op.cost;
-                work += op.work;
             } else if (op.perm) {
                 std::memset(blocked, 2, sizeof blocked);
-                open = 0;
             } else {
-                for (int k = 0; k < op.nq; ++k) {
-                    const char lv = op.diag[k] ? 1 : 2;
-                    open -= inB[op.q[k]] && !blocked[op.q[k]];
-                    blocked[op.q[k]] = std::max(blocked[op.q[k]], lv);
-                }
+                for (int k = 0; k < op.nq; ++k)
+                    blocked[op.q[k]] = std::max<char>(blocked[op.q[k]], op.diag[k] ? 1 : 2);
             }
-            if (!each(i, ok)) break;
-            if (!open && !grow) break;   // counting: no more work can join
+            each(i, ok);
+        }
+    }
+
+    // The same walk on tile bits B (a mask) that do not grow, for the work
+    // that joins alone: qubits as bits, up to where no more can.
+    struct Masks {
+        uint64_t diag, other, tile;   // qubits it is diagonal on, its other qubits, tile bits
+        uint16_t cost;
+        uint8_t work, perm;
+    };
+    static size_t count(const std::vector<Masks> &pending, uint64_t B, size_t lim) {
+        uint64_t left = 0, left_other = 0;   // qubits of ops left out / of those not diagonal there
+        size_t used = 256, work = 0;
+        for (const Masks &op : pending) {
+            if (!op.perm && !(left_other & op.diag) && !(left & op.other) && !(op.tile & ~B) &&
+                (used == 256 || used + op.cost <= lim)) {
+                used += op.cost;
+                work += op.work;
+                continue;
+            }
+            if (op.perm) break;
+            left |= op.diag | op.other;
+            left_other |= op.other;
+            if (!(B & ~left)) break;
         }
         return work;
     }
@@ -613,28 +643,39 @@ struct Builder {
     // Tile bits grown ahead: the first ops' bits, then one at a time the
     // qubit of the next pending ops that lets the most work join.
     void choose_tile(const std::vector<size_t> &pending, std::vector<char> &inB, int &nB) const {
-        auto none = [](size_t, bool) { return true; };
-        size_t base = walk(pending, inB, nullptr, none);
+        std::vector<Masks> masks(pending.size());
+        for (size_t j = 0; j < pending.size(); ++j) {
+            const Lite &op = lite[pending[j]];
+            Masks &m = masks[j];
+            m = {0, 0, 0, op.cost, op.work, op.perm};
+            for (int k = 0; k < op.nq; ++k) (op.diag[k] ? m.diag : m.other) |= 1ull << op.q[k];
+            for (int k = 0; k < op.nb; ++k) m.tile |= 1ull << op.b[k];
+        }
+        uint64_t B = 0;
+        for (int q = 0; q < n; ++q) B |= (uint64_t)(inB[q] != 0) << q;
+        const size_t lim = budget();
+        size_t base = count(masks, B, lim);
         while (nB < T) {
-            std::vector<char> cand(n, 0);
-            std::vector<int> cands;
+            int cands[64], ncands = 0;
+            uint64_t cand = B;
             for (size_t j = 0, seen = 0; j < pending.size() && seen < 64; ++j) {
                 const Lite &op = lite[pending[j]];
                 seen += op.nb > 0;
-                for (int k = 0; k < op.nb; ++k)
-                    if (!inB[op.b[k]] && !cand[op.b[k]]) cand[op.b[k]] = 1, cands.push_back(op.b[k]);
+                for (int k = 0; k < op.nb; ++k) {
+                    if (!((cand >> op.b[k]) & 1)) cands[ncands++] = op.b[k];
+                    cand |= 1ull << op.b[k];
+                }
             }
-            if (cands.empty()) break;
+            if (!ncands) break;
             int best = -1;
             size_t bestc = base;
-            for (int q : cands) {
-                inB[q] = 1;
-                const size_t c = walk(pending, inB, nullptr, none);
-                inB[q] = 0;
-                if (c > bestc) best = q, bestc = c;
+            for (int k = 0; k < ncands; ++k) {
+                const size_t c = count(masks, B | 1ull << cands[k], lim);
+                if (c > bestc) best = cands[k], bestc = c;
             }
             if (best < 0) best = cands[0];   // the earliest: a later choice may need it
             inB[best] = 1;
+            B |= 1ull << best;
             ++nB;
             base = bestc;
         }
@@ -647,9 +688,7 @@ struct Builder {
     };
     std::vector<Part> parts = {};
     int partition() {
-        make_lite();
-        std::vector<size_t> pending(ops.size()), rest;
-        for (size_t i = 0; i < ops.size(); ++i) pending[i] = i;
+        std::vector<size_t> pending = list.order[asap], rest;
         while (!pending.empty()) {
             Part p;
             if (lite[pending[0]].perm) {
@@ -665,7 +704,6 @@ struct Builder {
             rest.clear();
             walk(pending, inB, &nB, [&](size_t i, bool ok) {
                 (ok ? p.take : rest).push_back(i);
-                return true;
             });
             if (p.take.empty())
                 return fail(QK_ERR_ARG, "tile_bits %d: an operation needs %d tile qubits", T, lite[pending[0]].nb);
@@ -680,13 +718,14 @@ struct Builder {
         return QK_OK;
     }
 
-    int compile_parts() {
+    // limit: give up (plan.nremaps at least that) where the plan is no better
+    int compile_parts(size_t limit) {
         size_t last = parts.size();   // the last compute pass
         while (last && parts[last - 1].B.empty()) --last;
         for (size_t k = 0; k < parts.size(); ++k) {
             if (!parts[k].B.empty()) {
-                int rc = compile(parts[k].take, parts[k].B, k + 1 == last);
-                if (rc) return rc;
+                int rc = compile(parts[k].take, parts[k].B, k + 1 == last, limit);
+                if (rc || plan.nremaps >= limit) return rc;
                 continue;
             }
             flush();
@@ -731,19 +770,29 @@ struct Builder {
         for (size_t k = 0; k < take.size(); ++k)
             (keep[k] ? t2 : rest).push_back(take[k]);
         take.swap(t2);
-        std::sort(rest.begin(), rest.end());
+        std::sort(rest.begin(), rest.end(), [&](size_t a, size_t b) { return list.rank[asap][a] < list.rank[asap][b]; });
     }
 
     // ---- one pass ----
+    struct Span {
+        const int *b, *e;
+        const int *begin() const { return b; }
+        const int *end() const { return e; }
+    };
     struct Pass {
         std::vector<size_t> idx;
         std::vector<int> work;       // positions of unitaries and gradients not yet done
-        std::vector<std::vector<int>> preds;
+        std::vector<int> other;      // and of the others
+        std::vector<int> pred_list, pred0;   // op k's predecessors: pred_list[pred0[k] .. pred0[k + 1])
+        Span preds(int k) const { return {pred_list.data() + pred0[k], pred_list.data() + pred0[k + 1]}; }
         std::vector<char> done;
         std::vector<int> local, Q;   // state bit -> tile bit or -1; slots (tile bits, ascending)
+        uint32_t qmask = 0;          // the bits of Q
         std::vector<int> outer;      // state bit outside the tile -> bit of the tile number
         std::vector<char> dirty;     // per state bit: 1 CX control, 2 label changed since the re-mapping
         size_t left = 0, work_left = 0;
+        std::vector<int> head, next_work;   // a qubit's work in order: the first, and after each the next, or -1
+        std::vector<int> phases;            // (of mark_work)
     };
 
     int slot(const Pass &P, int q) const {
@@ -752,47 +801,40 @@ struct Builder {
         const auto it = std::find(P.Q.begin(), P.Q.end(), b);
         return it == P.Q.end() ? -1 : (int)(it - P.Q.begin());
     }
+    bool is_slot(const Pass &P, int q) const { return P.local[q] >= 0 && ((P.qmask >> P.local[q]) & 1); }
     bool is_phase(const Op &op) const { return op.kind == OP_PHASE1 || op.kind == OP_PHASE2; }
     bool is_phase(const Lite &op) const { return !op.nb && !op.perm; }
 
     // Undone predecessors of op k that are phases which can run now; false
     // when another predecessor is undone.
-    bool pending_phases(const Pass &P, const std::vector<char> &done, int k, std::vector<int> *out) const {
-        if (out) out->clear();
-        for (int p : P.preds[k]) {
-            if (done[p]) continue;
+    bool pending_phases(const Pass &P, int k, std::vector<int> *out) const {
+        out->clear();
+        for (int p : P.preds(k)) {
+            if (P.done[p]) continue;
             const Lite &o = lite[P.idx[p]];
             if (!is_phase(o)) return false;
             for (int j = 0; j < o.nq; ++j)
                 if (P.dirty[o.q[j]] > 1) return false;
-            for (int pp : P.preds[p])
-                if (!done[pp]) return false;
-            if (out) out->push_back(p);
+            for (int pp : P.preds(p))
+                if (!P.done[pp]) return false;
+            out->push_back(p);
         }
         return true;
     }
 
-    // Run (emit) or count the work that can run under slots P.Q.
-    size_t run_work(Pass &P, bool emit) {
-        std::vector<char> copy;
-        if (!emit) copy = P.done;
-        std::vector<char> &done = emit ? P.done : copy;
+    // Run (emit) the work that can run under slots P.Q.
+    void run_work(Pass &P) {
         std::vector<int> ph;
-        size_t cnt = 0;
-        bool trim = false;
         for (bool progress = true; progress;) {
             progress = false;
             for (int k : P.work) {
                 const int q = lite[P.idx[k]].q[0];
-                if (done[k] || slot(P, q) < 0 || P.dirty[q]) continue;
-                if (!pending_phases(P, done, k, &ph)) continue;
+                if (P.done[k] || !is_slot(P, q) || P.dirty[q]) continue;
+                if (!pending_phases(P, k, &ph)) continue;
                 const Op &op = ops[P.idx[k]];
-                for (int p : ph) done[p] = 1;
-                done[k] = 1;
-                ++cnt;
+                for (int p : ph) P.done[p] = 1;
+                P.done[k] = 1;
                 progress = true;
-                if (!emit) continue;
-                trim = true;
                 P.left -= 1 + ph.size();
                 --P.work_left;
                 if (op.kind == OP_K) emit_k(P, op, ph);
@@ -802,8 +844,35 @@ struct Builder {
                 }
             }
         }
-        if (trim)
-            P.work.erase(std::remove_if(P.work.begin(), P.work.end(), [&](int k) { return P.done[k] != 0; }), P.work.end());
+        trim(P, P.work);
+    }
+    static void trim(const Pass &P, std::vector<int> &list) {
+        list.erase(std::remove_if(list.begin(), list.end(), [&](int k) { return P.done[k] != 0; }), list.end());
+    }
+
+    // Mark done what can run when qubit q joins the slots among `slots`, under
+    // which nothing more can: q's next work, then what that lets run.  What is
+    // marked goes to `marked`; returns the number of unitaries and gradients.
+    size_t mark_work(Pass &P, std::vector<int> &slots, int q, std::vector<int> &marked) const {
+        size_t cnt = 0;
+        auto run_queue = [&](int x) {   // x's work, in order
+            size_t before = cnt;
+            for (int k = P.head[x]; k >= 0; k = P.next_work[k]) {
+                if (P.done[k]) continue;
+                if (P.dirty[x] || !pending_phases(P, k, &P.phases)) break;
+                for (int p : P.phases) P.done[p] = 1, marked.push_back(p);
+                P.done[k] = 1;
+                marked.push_back(k);
+                ++cnt;
+            }
+            return cnt != before;
+        };
+        if (!run_queue(q)) return 0;
+        for (bool progress = true; progress;) {
+            progress = false;
+            for (int x : slots) progress = run_queue(x) || progress;
+            progress = run_queue(q) || progress;
+        }
         return cnt;
     }
 
@@ -813,18 +882,18 @@ struct Builder {
         std::vector<int> ph;
         for (bool progress = true; progress;) {
             progress = false;
-            for (size_t k = 0; k < P.idx.size(); ++k) {
+            for (int k : P.other) {
+                if (P.done[k]) continue;
                 const Op &op = ops[P.idx[k]];
-                if (P.done[k] || is_work(op)) continue;
                 if (is_phase(op)) {
                     if (P.work_left) continue;
                     bool ok = true;
                     for (int j = 0; j < op.nq; ++j) ok = ok && P.dirty[op.q[j]] < 2;
-                    for (int p : P.preds[k]) ok = ok && P.done[p];
+                    for (int p : P.preds(k)) ok = ok && P.done[p];
                     if (!ok) continue;
                     emit_phase(P, op);
                 } else {
-                    if (!pending_phases(P, P.done, (int)k, &ph)) continue;
+                    if (!pending_phases(P, k, &ph)) continue;
                     for (int p : ph) {
                         emit_phase(P, ops[P.idx[p]]);
                         P.done[p] = 1;
@@ -850,6 +919,7 @@ struct Builder {
                 progress = true;
             }
         }
+        trim(P, P.other);
         return changed;
     }
 
@@ -915,6 +985,8 @@ struct Builder {
     void remap(Pass &P, const std::vector<int> &Q, bool dirty) {
         P.Q = Q;
         std::sort(P.Q.begin(), P.Q.end());
+        P.qmask = 0;
+        for (int b : P.Q) P.qmask |= 1u << b;
         std::fill(P.dirty.begin(), P.dirty.end(), 0);
         TOp &t = step(TOP_REMAP);
         t.nbits = 1;
@@ -1067,25 +1139,35 @@ struct Builder {
     // lowest L bits to the threads (runs of contiguous amplitudes).
     std::vector<int> choose_slots(Pass &P, bool first, int lo) {
         std::vector<int> cand, Q;
+        uint32_t seen = first ? (1u << lo) - 1 : 0;
         for (int k : P.work) {
             const int b = P.local[lite[P.idx[k]].q[0]];
-            if ((!first || b >= lo) && std::find(cand.begin(), cand.end(), b) == cand.end()) cand.push_back(b);
+            if (!((seen >> b) & 1)) cand.push_back(b);
+            seen |= 1u << b;
+            if (seen + 1 == 1u << T) break;
         }
-        size_t base = 0;
+        std::vector<int> qubits(T), slots, all, marked;   // state bits of the tile bits / of Q; what is marked done
+        for (int q = 0; q < n; ++q)
+            if (P.local[q] >= 0) qubits[P.local[q]] = q;
+        auto undo = [&](std::vector<int> &m) {
+            for (int k : m) P.done[k] = 0;
+            m.clear();
+        };
         while ((int)Q.size() < r && !cand.empty()) {
-            int best = -1;
-            size_t bestc = base;
+            int best = 0;
+            size_t bestc = 0;
             for (size_t i = 0; i < cand.size(); ++i) {
-                P.Q = Q;
-                P.Q.push_back(cand[i]);
-                const size_t c = run_work(P, false);
+                const size_t c = mark_work(P, slots, qubits[cand[i]], marked);
+                undo(marked);
                 if (c > bestc) best = (int)i, bestc = c;
             }
-            if (best < 0) best = 0;
+            const int q = qubits[cand[best]];
+            if (bestc) mark_work(P, slots, q, all);
+            slots.push_back(q);
             Q.push_back(cand[best]);
             cand.erase(cand.begin() + best);
-            base = bestc;
         }
+        undo(all);
         fill_high(Q);
         return Q;
     }
@@ -1094,7 +1176,7 @@ struct Builder {
             if (std::find(Q.begin(), Q.end(), b) == Q.end()) Q.push_back(b);
     }
 
-    int compile(const std::vector<size_t> &idx, const std::vector<int> &B, bool last_pass) {
+    int compile(const std::vector<size_t> &idx, const std::vector<int> &B, bool last_pass, size_t limit) {
         PassDesc d;
         std::memset(&d, 0, sizeof d);
         d.form = 1;
@@ -1110,28 +1192,39 @@ struct Builder {
             if (P.local[q] < 0) P.outer[q] = k++;
         P.dirty.assign(n, 0);
         P.done.assign(idx.size(), 0);
-        P.preds.resize(idx.size());
+        P.pred0.reserve(idx.size() + 1);
+        P.pred0.push_back(0);
+        P.pred_list.reserve(3 * idx.size());
         P.left = idx.size();
         // predecessors: ops that share a qubit and are not both diagonal on it
         std::vector<int> lastn(n, -1);
         std::vector<std::vector<int>> diags(n);
         for (size_t k = 0; k < idx.size(); ++k) {
             const Op &op = ops[idx[k]];
-            if (is_work(op)) P.work.push_back((int)k);
+            (is_work(op) ? P.work : P.other).push_back((int)k);
             P.work_left += is_work(op);
             for (int j = 0; j < op.nq; ++j) {
                 const int q = op.q[j];
-                if (lastn[q] >= 0) P.preds[k].push_back(lastn[q]);
+                if (lastn[q] >= 0) P.pred_list.push_back(lastn[q]);
                 if (diagonal_on(op, q)) {
                     diags[q].push_back((int)k);
                 } else {
-                    P.preds[k].insert(P.preds[k].end(), diags[q].begin(), diags[q].end());
+                    P.pred_list.insert(P.pred_list.end(), diags[q].begin(), diags[q].end());
                     diags[q].clear();
                     lastn[q] = (int)k;
                 }
             }
-            std::sort(P.preds[k].begin(), P.preds[k].end());
-            P.preds[k].erase(std::unique(P.preds[k].begin(), P.preds[k].end()), P.preds[k].end());
+            const auto mine = P.pred_list.begin() + P.pred0.back();
+            std::sort(mine, P.pred_list.end());
+            P.pred_list.erase(std::unique(mine, P.pred_list.end()), P.pred_list.end());
+            P.pred0.push_back((int)P.pred_list.size());
+        }
+        P.head.assign(n, -1);
+        P.next_work.assign(idx.size(), -1);
+        for (size_t i = P.work.size(); i-- > 0;) {
+            const int k = P.work[i], q = ops[idx[k]].q[0];
+            P.next_work[k] = P.head[q];
+            P.head[q] = k;
         }
         d.prog0 = (int)plan.ops.size();
         d.coef0 = (int)(plan.coef.size() / 2);
@@ -1142,9 +1235,10 @@ struct Builder {
         remap(P, choose_slots(P, true, lo), false);
         for (bool first = true;; first = false) {
             const size_t before = P.left;
-            run_work(P, true);
+            run_work(P);
             dirty = run_labels(P) || dirty;
             if (!P.left) break;
+            if (plan.nremaps >= limit) return QK_OK;
             if (!first && P.left == before) return fail(QK_ERR_ARG, "planner: a pass makes no progress");
             remap(P, choose_slots(P, false, lo), dirty);
             dirty = false;
@@ -1155,10 +1249,10 @@ struct Builder {
             fill_high(Q);
             remap(P, Q, dirty);
         }
-        if (scaled && last_pass) {
+        if (list.scaled && last_pass) {
             TOp &t = step(TOP_SCALE);
             t.b = 1;
-            push(to_double(carry * tail));
+            push(to_double(carry * list.tail));
             carry = 1;
         }
         d.nprog = (int)plan.ops.size() - d.prog0;
@@ -1183,14 +1277,23 @@ struct Builder {
 // The candidates of a plan: op lists, each in both orders and with both ways
 // to choose tiles.  All are cut into passes; of those with the fewest passes
 // the first and the last are compiled, the one with fewer re-mappings kept.
-int build_best(const std::vector<std::vector<Op>> &lists, const std::vector<cl> &tail, const std::vector<char> &scaled,
-               int n, const PlanOptions &o, int nstates, HostPlan &plan) {
+int build_best(std::vector<List> lists, int n, const PlanOptions &o, int nstates, HostPlan &plan) {
     PlanOptions fo = o;
     fo.tile_bits = o.f_tile_bits;
     const int L = pass_low_bits(fo, n);
+    for (List &list : lists) {
+        make_lite(list, o.dtype == QK_C128 ? 16 : 8, o.f_tile_bits - o.f_reg_bits);
+        list.order[0].resize(list.ops.size());
+        for (size_t i = 0; i < list.ops.size(); ++i) list.order[0][i] = i;
+        list.order[1] = asap_positions(list.ops, n);
+        for (int k = 0; k < 2; ++k) {
+            list.rank[k].resize(list.ops.size());
+            for (size_t i = 0; i < list.ops.size(); ++i) list.rank[k][list.order[k][i]] = i;
+        }
+    }
     struct Candidate {
         size_t list = 0;
-        std::vector<Op> ops;
+        bool asap = false;
         std::vector<Builder::Part> parts;
     } first, last;
     HostPlan empty;
@@ -1199,21 +1302,24 @@ int build_best(const std::vector<std::vector<Op>> &lists, const std::vector<cl> 
     empty.T = o.f_tile_bits;
     empty.r = o.f_reg_bits;
     empty.nstates = nstates;
-    std::vector<Candidate> all(4 * lists.size());
+    // (in one tile there is no choice of tiles)
+    const size_t variants = n <= o.f_tile_bits ? 2 : 4;
+    std::vector<Candidate> all(variants * lists.size());
+    auto builder = [&](const Candidate &c, bool lookahead, HostPlan &hp) {
+        return Builder{lists[c.list], c.asap, n, o.f_tile_bits, o.f_reg_bits, L, hp, o, lookahead};
+    };
     auto candidate = [&](size_t k) {
-        const size_t list = k / 4, variant = k % 4;
         Candidate &c = all[k];
-        c.list = list;
-        c.ops = lists[list];
-        if (variant % 2) asap_order(c.ops, n);
+        c.list = k / variants;
+        c.asap = k % 2;
         HostPlan hp = empty;
-        Builder b{c.ops, n, o.f_tile_bits, o.f_reg_bits, L, hp, o, variant >= 2, tail[list], scaled[list] != 0};
+        Builder b = builder(c, k % variants >= 2, hp);
         const int rc = b.partition();
         c.parts.swap(b.parts);
         return rc;
     };
-    // (a thread costs some 30 us to start, a candidate of a few hundred ops more)
-    const bool threads = o.threads && lists[0].size() >= 100;
+    // (threads take longer to start than candidates of fewer ops)
+    const bool threads = o.threads && variants == 4 && lists[0].ops.size() >= 300;
     for (size_t k = 0; k < all.size() && !threads; ++k) {
         int rc = candidate(k);
         if (rc) return rc;
@@ -1232,10 +1338,9 @@ int build_best(const std::vector<std::vector<Op>> &lists, const std::vector<cl> 
     for (Candidate *c : {&first, &last}) {
         if (c == &last && !two) break;
         HostPlan hp = empty;
-        Builder b{c->ops, n, o.f_tile_bits, o.f_reg_bits, L, hp, o, false, tail[c->list], scaled[c->list] != 0};
-        b.make_lite();
+        Builder b = builder(*c, false, hp);
         b.parts.swap(c->parts);
-        int rc = b.compile_parts();
+        int rc = b.compile_parts(c == &first ? SIZE_MAX : plan.nremaps);
         if (rc) return rc;
         if (c == &first || hp.nremaps < plan.nremaps) plan = std::move(hp);
     }
@@ -1244,54 +1349,55 @@ int build_best(const std::vector<std::vector<Op>> &lists, const std::vector<cl> 
 
 }  // namespace
 
-bool plan_is_factored(const qk_gate *gates, size_t ng, int n, const PlanOptions &o, int nstates) {
+// The gates lowered, where a factored program can run them.
+static bool lower_factored(const qk_gate *gates, size_t ng, int n, const PlanOptions &o, int nstates, std::vector<Op> *ops) {
     if (!sizes_fit(o, n, nstates)) return false;
     for (size_t i = 0; i < ng; ++i) {
         Op op;
         if (!factorable(gates[i], op)) return false;
         for (int k = 0; k < op.nq; ++k)
             if (op.q[k] < 0 || op.q[k] >= n) return false;
+        if (ops) ops->push_back(op);
     }
     return true;
+}
+
+bool plan_is_factored(const qk_gate *gates, size_t ng, int n, const PlanOptions &o, int nstates) {
+    return lower_factored(gates, ng, n, o, nstates, nullptr);
 }
 
 static int forward(const qk_gate *gates, size_t ng, int n, const PlanOptions &o, HostPlan &plan) {
     int rc = check_options(o, n);
     if (rc) return rc;
-    if (!plan_is_factored(gates, ng, n, o, 1)) return build_plan(gates, ng, n, o, plan);
-    std::vector<Op> lowered(ng);
+    std::vector<Op> lowered;
+    lowered.reserve(ng);
+    if (!lower_factored(gates, ng, n, o, 1, &lowered)) return build_plan(gates, ng, n, o, plan);
     bool swaps = false;
-    for (size_t i = 0; i < ng; ++i) {
-        factorable(gates[i], lowered[i]);
-        swaps = swaps || (lowered[i].kind == OP_SWAP2 && lowered[i].aux != 1);
-    }
+    for (const Op &op : lowered) swaps = swaps || (op.kind == OP_SWAP2 && op.aux != 1);
     // SWAP gates as label steps, or as renamings too
-    std::vector<std::vector<Op>> lists;
-    std::vector<cl> tail;
-    std::vector<char> scaled;
-    for (int rename = 0; rename <= (swaps ? 1 : 0); ++rename) {
-        std::vector<Op> ops = lowered;
-        relabel_perms(ops, n, pass_low_bits(o, n), perm_tile_bits(o.dtype), 6, rename);
-        merge_runs(ops, n);
-        cl f;
-        bool has;
-        factor(ops, n, o, f, has);
-        lists.push_back(std::move(ops));
-        tail.push_back(f);
-        scaled.push_back(has);
+    std::vector<List> lists(swaps ? 2 : 1);
+    for (size_t k = 0; k < lists.size(); ++k) {
+        List &l = lists[k];
+        if (k + 1 < lists.size()) l.ops = lowered;
+        else l.ops = std::move(lowered);
+        relabel_perms(l.ops, n, pass_low_bits(o, n), perm_tile_bits(o.dtype), 6, k > 0);
+        merge_runs(l.ops, n);
+        factor(l.ops, n, o, l.tail, l.scaled);
     }
-    return build_best(lists, tail, scaled, n, o, 1, plan);
+    return build_best(std::move(lists), n, o, 1, plan);
 }
 
 static int adjoint(const qk_gate *gates, size_t ng, const int32_t *pidx, int n, const PlanOptions &o, HostPlan &plan) {
     int rc = check_options(o, n);
     if (rc) return rc;
-    if (!plan_is_factored(gates, ng, n, o, 2)) return build_adjoint_plan(gates, ng, pidx, n, o, plan);
-    std::vector<Op> ops;
+    std::vector<Op> lowered;
+    lowered.reserve(ng);
+    if (!lower_factored(gates, ng, n, o, 2, &lowered)) return build_adjoint_plan(gates, ng, pidx, n, o, plan);
+    std::vector<List> lists(1);
+    std::vector<Op> &ops = lists[0].ops;
     ops.reserve(2 * ng);
     for (size_t i = ng; i-- > 0;) {
-        Op op;
-        factorable(gates[i], op);
+        Op &op = lowered[i];
         if (pidx && pidx[i] >= 0) {
             const int gen = gates[i].kind == QK_GATE_RX ? 1 : gates[i].kind == QK_GATE_RY ? 2 : gates[i].kind == QK_GATE_RZ ? 3 : 0;
             if (!gen) return fail(QK_ERR_UNSUPPORTED, "gate %zu: only RX, RY, RZ are trainable", i);
@@ -1310,10 +1416,8 @@ static int adjoint(const qk_gate *gates, size_t ng, const int32_t *pidx, int n, 
     hoist_gradients(ops, n);
     merge_runs(ops, n);
     pair_gradients(ops);
-    cl tail;
-    bool scaled;
-    factor(ops, n, o, tail, scaled);
-    return build_best({ops}, {tail}, {scaled}, n, o, 2, plan);
+    factor(ops, n, o, lists[0].tail, lists[0].scaled);
+    return build_best(std::move(lists), n, o, 2, plan);
 }
 
 int plan_forward(const qk_gate *gates, size_t ng, int n, const PlanOptions &o, HostPlan &plan) {

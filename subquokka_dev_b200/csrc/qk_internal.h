@@ -247,6 +247,7 @@ bool one_qubit(const Op &op);
 void as_matrix(const Op &op, double (&m)[8]);
 void mat2_mul(const double (&x)[8], const double (&y)[8], double (&z)[8]);
 void asap_order(std::vector<Op> &ops, int n);
+std::vector<size_t> asap_positions(const std::vector<Op> &ops, int n);   // the ops in that order
 void merge_one_qubit_runs(std::vector<Op> &ops, int n);
 void absorb_into_two_qubit_ops(std::vector<Op> &ops, int n, bool keep_real = false);
 bool op_is_real(const Op &op);

@@ -18,7 +18,7 @@ namespace qk {
 // ASAP layers: level = 1 + the highest level on the op's qubits (a
 // permutation op takes every qubit's level); a stable sort by level keeps
 // each qubit's op order, so the list computes the same state.
-void asap_order(std::vector<Op> &ops, int n) {
+std::vector<size_t> asap_positions(const std::vector<Op> &ops, int n) {
     std::vector<int> lvl(n, 0);
     std::vector<std::pair<int, size_t>> key(ops.size());
     for (size_t i = 0; i < ops.size(); ++i) {
@@ -30,10 +30,17 @@ void asap_order(std::vector<Op> &ops, int n) {
         for (int k = 0; k < (all ? n : op.nq); ++k) lvl[all ? k : op.q[k]] = l;
         key[i] = {l, i};
     }
-    std::stable_sort(key.begin(), key.end());
+    std::sort(key.begin(), key.end());
+    std::vector<size_t> at;
+    at.reserve(ops.size());
+    for (const auto &k : key) at.push_back(k.second);
+    return at;
+}
+
+void asap_order(std::vector<Op> &ops, int n) {
     std::vector<Op> sorted;
     sorted.reserve(ops.size());
-    for (const auto &k : key) sorted.push_back(ops[k.second]);
+    for (size_t i : asap_positions(ops, n)) sorted.push_back(ops[i]);
     ops.swap(sorted);
 }
 

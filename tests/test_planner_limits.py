@@ -1,4 +1,5 @@
-"""Planner calls that have no plan end with an error, and soon (CPU)."""
+"""Planner calls that have no plan end with an error, and soon; planning time
+(CPU)."""
 import os
 import shutil
 import subprocess
@@ -42,11 +43,12 @@ def test_one_qubit_tiles_take_what_needs_one():
 
 
 @pytest.mark.skipif(shutil.which("g++") is None, reason="g++ absent")
-def test_failed_allocations_are_errors(tmp_path):
+@pytest.mark.parametrize("check,opt", [("alloc_check", "-O1"), ("plan_time_check", "-O2")])
+def test_planner_check(check, opt, tmp_path):
     csrc = os.path.join(ROOT, "subquokka_dev_b200", "csrc")
-    exe = tmp_path / "alloc_check"
-    cmd = ["g++", "-O1", "-std=c++17", "-I", os.path.join(ROOT, "include"), "-I", csrc, "-I", os.path.join(ROOT, "tests"),
-           os.path.join(ROOT, "tests", "alloc_check.cpp")]
+    exe = tmp_path / check
+    cmd = ["g++", opt, "-std=c++17", "-I", os.path.join(ROOT, "include"), "-I", csrc, "-I", os.path.join(ROOT, "tests"),
+           os.path.join(ROOT, "tests", check + ".cpp")]
     cmd += [os.path.join(csrc, f) for f in ("qk_factor.cpp", "qk_plan.cpp", "qk_rewrite.cpp", "qk_parse.cpp", "qk_dense_host.cpp")]
     build = subprocess.run(cmd + ["-o", str(exe), "-lpthread"], capture_output=True, text=True)
     assert build.returncode == 0, build.stderr
