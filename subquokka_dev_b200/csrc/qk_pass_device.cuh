@@ -39,11 +39,14 @@ constexpr int pass_max_threads() {
 // thread) hold this many CTAs an SM; 0: there is none.  complex128, one state:
 // three, 168 registers instead of 241, 12 warps an SM instead of 8 (0.645 ->
 // 0.600 s on the 30-qubit random circuit).  complex64, two states: three, 168
-// registers instead of 254, and one state: five, 96 instead of 128 (26-qubit
-// HEA sweep 100.5 -> 89.9 ms; six CTAs of one state 90.4).
+// registers instead of 254 (26-qubit HEA sweep 100.5 -> 89.9 ms).  complex64,
+// one state: four, 128 registers: 28 qubits, 8 layers of dense two-qubit gates
+// 34.1 ms (34.2 without the instance; five CTAs, 96 registers and spills in the
+// 4x4 steps, 36.1), 300 mixed gates 47.2 (46.9; 49.7), 23-qubit 10-layer HEA
+// gradient 10.9 with either.
 template <typename C, int R, int NS>
 constexpr int pass_narrow_ctas() {
-    return R != 16 ? 0 : sizeof(C) == 16 ? (NS == 1 ? 3 : 0) : NS == 1 ? 5 : 3;
+    return R != 16 ? 0 : sizeof(C) == 16 ? (NS == 1 ? 3 : 0) : NS == 1 ? 4 : 3;
 }
 
 // Scatter the low bits of v into the set bits of mask, lowest first.
