@@ -390,21 +390,34 @@ static int group_terms(const qk_pauli_term *terms, size_t nterms, int n, std::ve
 constexpr int kPauliTileBits = 8 + kTileSlots;
 static_assert(1 << (kPauliTileBits - kTileSlots) == kRedThreads, "elements a thread");
 
+// Whether <H> of a group that shares its tile with no other is faster from
+// k_pauli_expval.  A tile pays for its shared-memory trip and set-up with the
+// signs of many terms (27 qubits, 32 terms: 3.9 -> 1.8 ms) or, in complex128,
+// with partners that a sweep reads a second time (one term, top qubit: 0.73 ->
+// 0.44 ms).  States of L2's size, microseconds flat / by tile: 20 qubits, one
+// term 27 / 29 to 28 / 36, 8 terms 38 / 40, 16 terms 53 / 43; 14 qubits, one
+// term 25 / 27, 32 terms 36 / 46.  Above, complex64, 25 qubits: one term 111 /
+// 123, two 148 / 136.
+static bool flat_alone(int nterms, int n, int dtype) {
+    const uint64_t bytes = (dtype == QK_C128 ? 16ull : 8ull) << n;
+    if (bytes <= 1ull << 20) return true;
+    if (bytes <= 16ull << 20) return nterms <= 8;
+    return dtype == QK_C64 && nterms == 1;
+}
+
 // The groups whose X masks fit a tile, cut into tiles; the others stay in
-// `flat` (one sweep each).
-static void tile_groups(const std::vector<PauliGroup> &groups, int n, int dtype, std::vector<PauliTile> &tiles,
-                        std::vector<PauliGroup> &flat) {
+// `flat` (one sweep each).  apply: for H psi, where <H> comes with the tiles.
+static void tile_groups(const std::vector<PauliGroup> &groups, int n, int dtype, bool apply, std::vector<PauliTile> &tiles,
+                        std::vector<const PauliGroup *> &flat) {
     const int T = std::min(n, kPauliTileBits), L = std::min(T, dtype == QK_C128 ? 3 : 4);   // 128-byte runs
     const uint64_t low = (1ull << L) - 1;
     std::vector<const PauliGroup *> left;
     for (const PauliGroup &g : groups) {
-        if (__builtin_popcountll(g.x | low) > T) flat.push_back(g);
+        if (__builtin_popcountll(g.x | low) > T) flat.push_back(&g);
         else left.push_back(&g);
     }
     std::stable_sort(left.begin(), left.end(), [](const PauliGroup *a, const PauliGroup *b) { return a->x < b->x; });
     while (!left.empty()) {
-        PauliTile t;
-        std::memset(&t, 0, sizeof t);
         uint64_t bits = low;
         std::vector<const PauliGroup *> take, rest;
         int nt = 0;
@@ -414,6 +427,13 @@ static void tile_groups(const std::vector<PauliGroup> &groups, int n, int dtype,
             (ok ? take : rest).push_back(g);
             if (ok) bits |= g->x, nt += g->nterms;
         }
+        left.swap(rest);
+        if (!apply && take.size() == 1 && flat_alone(take[0]->nterms, n, dtype)) {
+            flat.push_back(take[0]);
+            continue;
+        }
+        PauliTile t;
+        std::memset(&t, 0, sizeof t);
         for (int q = 0; __builtin_popcountll(bits) < T; ++q) bits |= 1ull << q;
         t.d.T = T;
         for (int q = 0, k = 0; q < n; ++q)
@@ -440,15 +460,14 @@ static void tile_groups(const std::vector<PauliGroup> &groups, int n, int dtype,
         }
         t.term0[t.ngroups] = (int16_t)k;
         tiles.push_back(t);
-        left.swap(rest);
     }
 }
 
-// out = H psi (out may be null) and, with acc (zero before), *acc = <H>.
+// Sweeps that H psi takes.
 static size_t pauli_sweeps(const std::vector<PauliGroup> &groups, int n, int dtype) {
     std::vector<PauliTile> tiles;
-    std::vector<PauliGroup> flat;
-    tile_groups(groups, n, dtype, tiles, flat);
+    std::vector<const PauliGroup *> flat;
+    tile_groups(groups, n, dtype, true, tiles, flat);
     return tiles.size() + flat.size();
 }
 
@@ -461,8 +480,8 @@ static int pauli_sum_t(C *out, const C *psi, int n, const std::vector<PauliGroup
         return e == cudaSuccess ? QK_OK : cuda_err(e, "memset");
     }
     std::vector<PauliTile> tiles;
-    std::vector<PauliGroup> flat;
-    tile_groups(groups, n, sizeof(C) == sizeof(double2) ? QK_C128 : QK_C64, tiles, flat);
+    std::vector<const PauliGroup *> flat;
+    tile_groups(groups, n, sizeof(C) == sizeof(double2) ? QK_C128 : QK_C64, out != nullptr, tiles, flat);
     constexpr bool c64 = sizeof(C) == sizeof(float2);
     const bool round = c64 && out, dot = out && acc && (round || !flat.empty());   // dot: <H> from all of H psi
     const auto kernel = round ? k_pauli_tile<C, c64> : k_pauli_tile<C, false>;
@@ -479,7 +498,8 @@ static int pauli_sum_t(C *out, const C *psi, int n, const std::vector<PauliGroup
         e = cudaGetLastError();
         if (e != cudaSuccess) return cuda_err(e, "k_pauli_tile");
     }
-    for (const PauliGroup &g : flat) {
+    for (const PauliGroup *gp : flat) {
+        const PauliGroup &g = *gp;
         if (out) k_pauli_apply<C><<<red_grid(namp), kRedThreads, 0, st>>>(out, psi, namp, g, done++ > 0);
         else k_pauli_expval<C><<<red_grid(namp), kRedThreads, 0, st>>>(psi, namp, g, acc);
     }
