@@ -70,12 +70,30 @@ int run_tasks(size_t n, const std::function<int(size_t)> &task) {
 // 25.0 against 23.9 ms, with 8 amplitudes a thread the brick takes 91 ms.
 // complex64: 4096-amplitude tiles, 32 amplitudes a thread: 75 ms on the
 // 29-qubit brick circuit against 76 ms with 2048 and 84 ms with 16 amplitudes.
+// Up to 17 qubits (complex128 18) there are not tiles enough for that: 1024
+// amplitudes, 8 a thread, so that more warps share a tile's chain of steps.
+// Microseconds with the large shapes and with these, complex64: 16 qubits, 20
+// brick layers 104 / 86, 12 HEA layers 178 / 147 (general programs 137, 145);
+// 13 qubits 82 / 54 and 139 / 107 (94, 99); 19 qubits 139 / 162 and 229 / 262.
+// complex128: 16 qubits 122 / 98 and 187 / 158 (174, 167); 18 qubits 158 / 139
+// and 217 / 194 (203, 195); 19 qubits 198 / 201 and 279 / 279.  Between them,
+// complex64 with 18 qubits: 2048, 16 a thread, 132 / 105 and 216 / 181 (167,
+// 180).
+// complex128 plans of little work a pass are bound by HBM and take 2048
+// amplitudes where that means fewer passes (below 36 units a pass, a unitary
+// 4, a two-qubit phase 1): 27 qubits, a layer of H 3.12 -> 2.55 ms, 2 HEA
+// layers 9.54 -> 9.21 (general programs 10.3); above, 28 qubits, 12 HEA layers
+// (53 units) 97.5 -> 100.8.
+constexpr int kWideTileBits = 11;
+constexpr size_t kPassWork = 36;
 PlanOptions factored_plan_options(int dtype, int n) {
     PlanOptions o = default_plan_options(dtype, n);
-    o.f_tile_bits = std::min(n, dtype == QK_C128 ? 10 : 12);
-    o.f_reg_bits = std::min(o.f_tile_bits, dtype == QK_C128 ? 4 : 5);
+    const bool c128 = dtype == QK_C128, small = n <= (c128 ? 18 : 17), mid = !c128 && n == 18;
+    o.f_tile_bits = std::min(n, small || c128 ? 10 : mid ? 11 : 12);
+    o.f_reg_bits = std::min(o.f_tile_bits, small ? 3 : c128 || mid ? 4 : 5);
+    if (c128 && !small) o.f_wide_bits = kWideTileBits;
     o.f_flips = 1;
-    o.f_full = dtype == QK_C128;
+    o.f_full = c128;
     return o;
 }
 
@@ -1384,7 +1402,19 @@ static int forward(const qk_gate *gates, size_t ng, int n, const PlanOptions &o,
         merge_runs(l.ops, n);
         factor(l.ops, n, o, l.tail, l.scaled);
     }
-    return build_best(std::move(lists), n, o, 1, plan);
+    PlanOptions w = o;
+    w.f_tile_bits = o.f_wide_bits;
+    size_t work = 0;
+    for (const Op &op : lists[0].ops) work += op.kind == OP_K ? 4 : op.kind == OP_PHASE2;
+    const bool wide = o.f_wide_bits > o.f_tile_bits && sizes_fit(w, n, 1);
+    std::vector<List> again;
+    if (wide) again = lists;
+    rc = build_best(std::move(lists), n, o, 1, plan);
+    if (rc || !wide || work >= kPassWork * plan.passes.size()) return rc;
+    HostPlan other;
+    rc = build_best(std::move(again), n, w, 1, other);
+    if (!rc && other.passes.size() < plan.passes.size()) plan = std::move(other);
+    return rc;
 }
 
 static int adjoint(const qk_gate *gates, size_t ng, const int32_t *pidx, int n, const PlanOptions &o, HostPlan &plan) {

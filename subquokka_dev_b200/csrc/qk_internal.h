@@ -221,6 +221,7 @@ struct PlanOptions {
     // plan_forward / plan_adjoint: tile and register bits of factored programs,
     // which are made where they can be (0: general programs only)
     int f_tile_bits = 0, f_reg_bits = 0;
+    int f_wide_bits = 0;  // tile bits a forward plan takes instead where that means fewer passes of little work
     int f_flips = 0;      // 1: factored programs may flip a tile bit (TOP_LCX with kNoQubit); 0: two rotations instead
     int f_full = 0;       // 1: factored programs may hold layers of full unitaries (kLayerFull); 0: rotations only
     int threads = 0;      // 1: the factored planner tries its candidates on several host threads

@@ -409,7 +409,7 @@ int qk_plan_create(const qk_gate *gates, size_t n, int nqubits, const qk_plan_op
         return QK_OK;
     }
     PlanOptions o = factored_plan_options(dtype, nqubits);
-    if (opts && opts->tile_bits) o.tile_bits = o.f_tile_bits = opts->tile_bits;
+    if (opts && opts->tile_bits) o.tile_bits = o.f_tile_bits = opts->tile_bits, o.f_wide_bits = 0;
     if (opts && opts->reg_bits) o.reg_bits = o.f_reg_bits = opts->reg_bits;
     o.f_reg_bits = std::min(o.f_reg_bits, o.f_tile_bits);
     o.threads = 1;
@@ -439,7 +439,7 @@ int qk_plan_create_groups(const qk_gate *gates, const int32_t *group_sizes, size
     }
     const int dtype = opts ? opts->dtype : QK_C128;
     PlanOptions o = factored_plan_options(dtype, nqubits);
-    if (opts && opts->tile_bits) o.tile_bits = o.f_tile_bits = opts->tile_bits;
+    if (opts && opts->tile_bits) o.tile_bits = o.f_tile_bits = opts->tile_bits, o.f_wide_bits = 0;
     if (opts && opts->reg_bits) o.reg_bits = o.f_reg_bits = opts->reg_bits;
     o.f_reg_bits = std::min(o.f_reg_bits, o.f_tile_bits);
     o.threads = 1;

@@ -130,3 +130,24 @@ def test_gradients_of_circuits_with_h_and_x(n, dtype):
         sv.upload(init)
         ev, grad, _ = adjoint_grad(sv, circ, idx, k, terms, 2, True)
         assert abs(ev - ref[0]) <= tol and np.abs(grad - ref[1]).max() <= tol
+
+
+@pytest.mark.parametrize("n,passes", [(25, 3), (27, 3), (28, 4)])
+def test_plans_of_little_work_take_wide_tiles(n, passes):
+    # 2048-amplitude tiles with the three lowest qubits: eight more a pass
+    circ = Circuit([make_gate("H", [q]) for q in range(n)])
+    assert Plan(circ, n, "c128").stats()[0] == passes
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["c128", "c64"])
+@pytest.mark.parametrize("n", [17, 18, 19, 20])
+def test_tile_shapes_by_size(n, dtype):
+    # about the sizes where the shape changes; 200 gates of at most four
+    # roundings of the state's norm
+    init = circuits.random_state(n, 6)
+    tol = 200 * 4 * (2.0 ** -53 if dtype == "c128" else 2.0 ** -24)
+    for circ in (Circuit([make_gate(g, [q]) for g in "HX" for q in range(n)]), mixed_circuit(n, 200, n)):
+        ref = oracle.apply_circuit(init, n, circ)
+        for got in both_ways(circ, n, dtype, init):
+            assert np.linalg.norm(got - ref) <= tol
