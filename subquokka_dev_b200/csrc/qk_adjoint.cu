@@ -463,17 +463,21 @@ static void tile_groups(const std::vector<PauliGroup> &groups, int n, int dtype,
     }
 }
 
-// Sweeps that H psi takes.
-static size_t pauli_sweeps(const std::vector<PauliGroup> &groups, int n, int dtype) {
-    std::vector<PauliTile> tiles;
-    std::vector<const PauliGroup *> flat;
-    tile_groups(groups, n, dtype, true, tiles, flat);
-    return tiles.size() + flat.size();
-}
+// What a call of pauli_sum_t launched: sweeps over psi, and whether <H> was a
+// sweep of its own (k_dot_re).
+struct PauliSweeps {
+    int sums = 0;
+    bool dot = false;
+    int launches() const { return std::max(1, sums) + dot; }   // (an empty sum clears out)
+    // bytes of H psi on states of S bytes: psi read and out written, by every
+    // further sweep out read too; the dot reads both
+    double bytes(double S) const { return sums ? 2 * S + 3 * S * (sums - 1) + (dot ? 2 * S : 0) : S; }
+};
 
 // out = H psi (out may be null) and, with acc (zero before), *acc = <H>.
 template <typename C>
-static int pauli_sum_t(C *out, const C *psi, int n, const std::vector<PauliGroup> &groups, double *acc, cudaStream_t st) {
+static int pauli_sum_t(C *out, const C *psi, int n, const std::vector<PauliGroup> &groups, double *acc, cudaStream_t st,
+                       PauliSweeps *sweeps = nullptr) {
     const uint64_t namp = 1ull << n;
     if (groups.empty()) {
         cudaError_t e = out ? cudaMemsetAsync(out, 0, sizeof(C) * namp, st) : cudaSuccess;
@@ -484,6 +488,7 @@ static int pauli_sum_t(C *out, const C *psi, int n, const std::vector<PauliGroup
     tile_groups(groups, n, sizeof(C) == sizeof(double2) ? QK_C128 : QK_C64, out != nullptr, tiles, flat);
     constexpr bool c64 = sizeof(C) == sizeof(float2);
     const bool round = c64 && out, dot = out && acc && (round || !flat.empty());   // dot: <H> from all of H psi
+    if (sweeps) *sweeps = {(int)(tiles.size() + flat.size()), dot};
     const auto kernel = round ? k_pauli_tile<C, c64> : k_pauli_tile<C, false>;
     int done = 0;
     for (const PauliTile &t : tiles) {
@@ -551,7 +556,6 @@ static int adjoint_t(C *psi, int n, int dtype, const qk_gate *gates, size_t ng, 
     if (e == cudaSuccess) e = cudaEventRecord(ws.ev0, st);
     if (e != cudaSuccess) return cuda_err(e, "sweep timing events");
     ws.last_fwd = ws.last_bwd = (int)ng;   // one launch per gate each way
-    ws.last_other = (int)(pauli_sweeps(groups, n, dtype) + 3 * cpos.size());
     ws.last_bytes = 0;                     // not counted for the per-gate sweep
     e = cudaMemsetAsync(dacc, 0, nacc * sizeof(double), st);
     if (e != cudaSuccess) return cuda_err(e, "clear accumulators");
@@ -568,8 +572,10 @@ static int adjoint_t(C *psi, int n, int dtype, const qk_gate *gates, size_t ng, 
         if (rc) return rc;
     }
     // lambda = H psi, <H> = Re<psi|lambda>
-    rc = pauli_sum_t<C>(lam, psi, n, groups, dacc + nparams, st);
+    PauliSweeps hs;
+    rc = pauli_sum_t<C>(lam, psi, n, groups, dacc + nparams, st, &hs);
     if (rc) return rc;
+    ws.last_other = (int)(hs.launches() + 3 * cpos.size());
     // backward
     for (size_t i = ng; i-- > 0;) {
         Op inv = ops[i];
@@ -687,20 +693,11 @@ static int adjoint_fused_t(C *psi, int n, int dtype, const qk_gate *gates, size_
     if (e != cudaSuccess) return cuda_err(e, "sweep timing events");
     e = cudaMemsetAsync(dacc, 0, nacc * sizeof(double), st);
     if (e != cudaSuccess) return cuda_err(e, "clear accumulators");
-    // algorithmic traffic: a forward pass reads and writes psi (2S), a
-    // two-state pass psi and lambda (4S); lambda = H psi reads psi and writes
-    // lambda (2S) and every further Pauli group re-reads lambda (3S); <H>
-    // reads both (2S); each checkpoint copy, drift check and restore 2S
     ws.last_fwd = ws.last_bwd = ws.last_other = 0;
     for (size_t sgi = 0; sgi < nseg; ++sgi) {
         ws.last_fwd += (int)fwd[sgi].passes.size();
         ws.last_bwd += (int)bwd[sgi].passes.size();
     }
-    const double S = (double)bytes;
-    const double nh = (double)std::max<size_t>(1, pauli_sweeps(groups, n, dtype));
-    ws.last_other = (int)(nh + 3 * (nseg - 1));
-    ws.last_bytes = 2 * S * ws.last_fwd + 4 * S * ws.last_bwd + (groups.empty() ? S : 2 * S + 3 * S * (nh - 1)) +
-                    3 * 2 * S * (double)(nseg - 1);
     // forward
     for (size_t sgi = 0; sgi < nseg; ++sgi) {
         if (sgi > 0) {
@@ -710,8 +707,15 @@ static int adjoint_fused_t(C *psi, int n, int dtype, const qk_gate *gates, size_
         int rc = run_forward_plan(psi, fwd[sgi], ws.plans[2 * sgi], st);
         if (rc) return rc;
     }
-    int rc = pauli_sum_t<C>(lam, psi, n, groups, dacc + nparams, st);
+    PauliSweeps hs;
+    int rc = pauli_sum_t<C>(lam, psi, n, groups, dacc + nparams, st, &hs);
     if (rc) return rc;
+    // algorithmic traffic: a forward pass reads and writes psi (2S), a
+    // two-state pass psi and lambda (4S); each checkpoint copy, drift check
+    // and restore 2S
+    const double S = (double)bytes;
+    ws.last_other = (int)(hs.launches() + 3 * (nseg - 1));
+    ws.last_bytes = 2 * S * ws.last_fwd + 4 * S * ws.last_bwd + hs.bytes(S) + 3 * 2 * S * (double)(nseg - 1);
     // backward
     for (size_t sgi = nseg; sgi-- > 0;) {
         rc = run_adjoint_plan(psi, lam, dtype, bwd[sgi], ws.plans[2 * sgi + 1], dacc, st);
