@@ -75,7 +75,10 @@ class ParamCircuit:
         rec["q"][row, col] = np.fromiter((int(q) for g in qs for q in g), dtype=np.int32, count=row.size)
         rec["param"] = vals
         free = idx >= 0
-        rec["param"][free] = np.asarray(params, dtype=np.float64)[idx[free]]
+        if type(params) is np.ndarray and params.ndim == 1:
+            rec["param"][free] = params[idx[free]]
+        else:   # a list, a tensor, anything whose elements are numbers
+            rec["param"][free] = [float(params[p]) for p in idx[free].tolist()]
         flat = {}   # of this call's gates that share a matrix
         for i, c in enumerate(coeffs):
             if c is not None:
