@@ -26,8 +26,8 @@ template <typename C> __host__ __device__ __forceinline__ C mk(double re, double
 
 template <typename C> __device__ __forceinline__ C cmul(C a, C b) {
     C r;
-    r.x = a.x * b.x - a.y * b.y;
-    r.y = a.x * b.y + a.y * b.x;
+    r.x = fma(a.x, b.x, -a.y * b.y);
+    r.y = fma(a.x, b.y, a.y * b.x);
     return r;
 }
 
