@@ -1,13 +1,12 @@
-// Device building blocks of factored passes (k_fpass in qk_fpass.cu, the
-// batched k_fpass_batch in qk_batch.cu): the thread's part of a tile and the
-// step interpreter.  The steps are defined in qk_internal.h, made by
-// qk_factor.cpp.
+// Device building blocks of factored passes (k_fpass in qk_fpass.cu): the
+// thread's part of a tile and the step interpreter.  The steps are defined in
+// qk_internal.h, made by qk_factor.cpp.
 //
 // A thread's amplitudes are named by labels (tile indices): register element
 // kk of thread tid carries label tb ^ XOR of bm[s] over the set bits s of kk.
 // A re-mapping writes the registers to the exchange buffer at their labels
-// and reads those of the next mapping; the label steps of CX and SWAP gates
-// only change tb and bm.  Under the first mapping each thread loads its
+// and reads those of the next mapping; the label steps of CX, SWAP and X
+// gates only change tb and bm.  Under the first mapping each thread loads its
 // amplitudes from HBM, under the last it stores them there: both leave the
 // lowest state bits to the lanes, so the accesses are the tile's contiguous
 // runs and neither goes through the exchange buffer.
@@ -342,12 +341,10 @@ __device__ __forceinline__ void run_steps(C (&v)[R], C (&w)[NS == 2 ? R : 1], un
         case TOP_GRAD: {
             if constexpr (NS == 2) {
                 T g = 0, g2 = 0;
-                switch (a) {
+                switch (a) {   // (two states: three slots at most)
                 case 0: g = reg_grad<0>(v, w, (int)b, m, &g2); break;
                 case 1: g = reg_grad<1>(v, w, (int)b, m, &g2); break;
                 case 2: g = reg_grad<2>(v, w, (int)b, m, &g2); break;
-                case 3: g = reg_grad<3>(v, w, (int)b, m, &g2); break;
-                case 4: g = reg_grad<4>(v, w, (int)b, m, &g2); break;
                 }
                 const uint32_t NT = blockDim.x;
                 gsm[(op.y & 0xFFFF) * NT + tid] += (double)g;
