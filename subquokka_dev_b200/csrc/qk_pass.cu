@@ -384,6 +384,20 @@ int apply_perm_gate(void *state, int n, int dtype, const Op &op, cudaStream_t st
 void release_scratch_plan(DevPlan &dp) { dp.release(); }
 }  // namespace qk
 
+// The engine's options for a plan, with what the caller asks for instead.
+static PlanOptions plan_options(int dtype, int n, const qk_plan_opts *opts) {
+    PlanOptions o = factored_plan_options(dtype, n);
+    if (opts && opts->tile_bits) {
+        o.tile_bits = o.f_tile_bits = opts->tile_bits;
+        o.f_reg_bits = dtype == QK_C128 ? 4 : 5;
+        o.f_wide_bits = 0;
+    }
+    if (opts && opts->reg_bits) o.reg_bits = o.f_reg_bits = opts->reg_bits;
+    o.f_reg_bits = std::min(o.f_reg_bits, o.f_tile_bits);
+    o.threads = 1;
+    return o;
+}
+
 extern "C" {
 
 int qk_plan_create(const qk_gate *gates, size_t n, int nqubits, const qk_plan_opts *opts, qk_plan **out) {
@@ -408,11 +422,7 @@ int qk_plan_create(const qk_gate *gates, size_t n, int nqubits, const qk_plan_op
         *out = p;
         return QK_OK;
     }
-    PlanOptions o = factored_plan_options(dtype, nqubits);
-    if (opts && opts->tile_bits) o.tile_bits = o.f_tile_bits = opts->tile_bits, o.f_wide_bits = 0;
-    if (opts && opts->reg_bits) o.reg_bits = o.f_reg_bits = opts->reg_bits;
-    o.f_reg_bits = std::min(o.f_reg_bits, o.f_tile_bits);
-    o.threads = 1;
+    const PlanOptions o = plan_options(dtype, nqubits, opts);
     auto *p = new qk_plan();
     int rc = plan_forward(gates, n, nqubits, o, p->hp);
     if (rc) {
@@ -438,11 +448,7 @@ int qk_plan_create_groups(const qk_gate *gates, const int32_t *group_sizes, size
         return qk_plan_create(gates, ng, nqubits, opts, out);
     }
     const int dtype = opts ? opts->dtype : QK_C128;
-    PlanOptions o = factored_plan_options(dtype, nqubits);
-    if (opts && opts->tile_bits) o.tile_bits = o.f_tile_bits = opts->tile_bits, o.f_wide_bits = 0;
-    if (opts && opts->reg_bits) o.reg_bits = o.f_reg_bits = opts->reg_bits;
-    o.f_reg_bits = std::min(o.f_reg_bits, o.f_tile_bits);
-    o.threads = 1;
+    const PlanOptions o = plan_options(dtype, nqubits, opts);
     auto *p = new qk_plan();
     int rc = build_group_plan(gates, group_sizes, ngroups, nqubits, o, p->hp);
     if (rc) {
