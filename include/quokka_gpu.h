@@ -250,10 +250,13 @@ int qk_apply_gates_timed(qk_sv *sv, const qk_gate *gates, size_t n, float *gate_
 typedef struct qk_plan_opts {
     int32_t dtype;        /* qk_dtype of the states the plan runs on        */
     int32_t tile_bits;    /* qubits per shared-memory tile (at most 14;
-                             default 11, 10 / 12 for factored complex128 /
-                             complex64 programs: see qk_plan_create)        */
+                             default 11; 10 / 12 for factored complex128 /
+                             complex64 programs, 10 or 11 for states of up to
+                             18 qubits and 11 for complex128 plans of little
+                             work: see qk_plan_create)                      */
     int32_t reg_bits;     /* qubits held in registers per thread (at most 4;
-                             default 4, 5 for factored complex64 programs)  */
+                             default 4; 5 for factored complex64 programs, 3
+                             for states of up to 17 qubits, complex128 18)  */
     int32_t fuse_width;   /* 0: register passes.  5 or 6: gates fused into
                              dense unitaries on at most that many qubits
                              (FP64 on the host, padded to 6 qubits), each
@@ -279,7 +282,12 @@ typedef struct qk_plan qk_plan;
  * do SWAP gates when that gives fewer passes; a final permutation restores
  * the layout.  Circuits whose one-qubit gates are unitary and whose two-qubit
  * gates are diagonal, CNOT or SWAP run factored programs (a unitary as two
- * phases and a rotation, CNOT and SWAP as labels), others dense ones. */
+ * phases and a rotation, CNOT, SWAP and X as labels), others dense ones, at
+ * about half the speed.  A U1 matrix counts as unitary (times a scalar) to
+ * 4e-15: computed in double or written with 16 digits, not with 12 or in
+ * single precision; one that is not sends the whole circuit there.  Stored
+ * amplitudes grow by up to 2^16 (complex64) or 2^48 (complex128) between
+ * passes of a factored plan and must leave the type room for that. */
 int qk_plan_create(const qk_gate *gates, size_t n, int nqubits, const qk_plan_opts *opts, qk_plan **out);
 /* The plan of a subcircuit file that qk_apply_groups runs: the gates of all
  * groups fused as one list, VSWAPs as renamings of the qubits after them.

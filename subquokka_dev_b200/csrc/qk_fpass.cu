@@ -10,8 +10,9 @@
 // scheduler's FP64 pipe a warp (128 are the pipe's own), a re-mapping 512
 // cycles of the shared-memory pipe; the two add up to about three quarters of
 // the time, the rest is the latency of steps and loads that 16 warps an SM do
-// not cover.  The general programs took 131 ms, this one 65 (2.2 times the
-// time of its 23 passes' HBM traffic).  complex64, 29 qubits: 169 -> 71 ms,
+// not cover.  The general programs took 131 ms, this one 66 (2.2 times the
+// time of its 23 passes' HBM traffic) and 70 with the worst of its rounded
+// matrices in the full form.  complex64, 29 qubits: 169 -> 71 ms,
 // issue bound (64 % of the slots).  A tile's offset comes from the uniform
 // loop of pass_base: gathered over the lanes by two reductions it delayed the
 // loads (complex64 76 ms).

@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(kBlock) k_diag2(C *__restrict__ s, uint64_t na
 // d[bit qa + 2 bit qb].  Only amplitudes that some gate changes are read and
 // written; a qubit t in every gate's mask (t >= 0) halves the sweep.  On its
 // own a CP moves S / 2 bytes, so the k CPs of a QFT row take k S / 2, here S:
-// bound by HBM, or by launches where the state lives in L2 (20-qubit QFT, 220
+// bound by HBM, in long runs by issue too, or by launches where the state lives in L2 (20-qubit QFT, 220
 // gates, 52 launches: 0.95 -> 0.33 ms).
 constexpr int kRunGates = 32;
 template <typename C> struct DiagRun {
